@@ -137,11 +137,13 @@ int ShapeIndex(uint32_t threads, uint32_t smem) {
 
 namespace {
 
-// Copy of `nodes` with padding0 = 1 on nodes holding a coordinate outside the
-// traversal kernel's fast-division window (0 or 2^-40..2^40), 0 elsewhere.
-std::vector<ae_bvh_node> FlagNodes(const ae_bvh_node* nodes, uint32_t n) {
-    std::vector<ae_bvh_node> out(nodes, nodes + n);
-    for (auto& nd : out) {
+// `nodes` in the device order, with padding0 = 1 on nodes holding a
+// coordinate outside the traversal kernel's fast-division window (0 or
+// 2^-40..2^40), 0 elsewhere.
+std::vector<PairedNode> DeviceNodes(const ae_bvh_node* nodes, uint32_t n) {
+    std::vector<PairedNode> out(n);
+    for (uint32_t i = 0; i < n; i++) {
+        ae_bvh_node nd = nodes[i];
         const float* c = nd.leftAABB.min;
         bool ok = true;
         for (int k = 0; k < 12; k++) {
@@ -150,6 +152,7 @@ std::vector<ae_bvh_node> FlagNodes(const ae_bvh_node* nodes, uint32_t n) {
         }
         nd.padding0 = ok ? 0 : 1;
         nd.padding1 = 0;
+        out[i] = PairNode(nd);
     }
     return out;
 }
@@ -414,10 +417,15 @@ __global__ void selftest_division_kernel(uint64_t n, uint32_t seed, unsigned lon
         // nearly equal pair (a tiny difference); c = 0 would make o subnormal, outside the window
         if ((h5 & 7u) == 0 && c != 0.0f) o = __uint_as_float(__float_as_uint(c) ^ (h5 & 0xffu));
         const float d = selftest_float(h4, h5, -40, 39, false);
-        const float a = __fsub_rn(c, o);
-        const float ref = __fdiv_rn(a, d);
-        const float got = div_rn_from_rcp(a, d, __frcp_rn(d));
-        if (__float_as_uint(ref) != __float_as_uint(got) && !(ref == 0.0f && got == 0.0f)) bad++;
+        // both halves of the packed form: the pair itself and its mirror image, whose
+        // quotient is the same with the other sign
+        const float ref = __fdiv_rn(__fsub_rn(c, o), d), y = __frcp_rn(d);
+        const f32x2 got = slab_quotients(pack2(c, -c), pack2(-o, o), pack2(-d, -d), pack2(y, y));
+        const float lo = lo2(got), hi = -hi2(got);
+        const bool zero = ref == 0.0f;
+        if ((__float_as_uint(ref) != __float_as_uint(lo) && !(zero && lo == 0.0f)) ||
+            (__float_as_uint(ref) != __float_as_uint(hi) && !(zero && hi == 0.0f)))
+            bad++;
     }
     for (int off = 16; off > 0; off >>= 1) bad += __shfl_down_sync(0xffffffffu, bad, off);
     if ((threadIdx.x & 31u) == 0 && bad) atomicAdd(mismatches, bad);
@@ -538,8 +546,8 @@ ae_rt_status ae_rt_mesh_upload(ae_rt_ctx* ctx, const ae_bvh_node* nodes, uint32_
         if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
         return e;
     };
-    std::vector<ae_bvh_node> flagged = FlagNodes(nodes, n_nodes);
-    cudaError_t e = upload(&m.nodes, flagged.data(), size_t(n_nodes) * sizeof(ae_bvh_node));
+    const std::vector<PairedNode> paired = DeviceNodes(nodes, n_nodes);
+    cudaError_t e = upload(&m.nodes, paired.data(), size_t(n_nodes) * sizeof(PairedNode));
     if (e == cudaSuccess) e = upload(&m.tris, tris, size_t(n_tris) * sizeof(ae_bvh_triangle));
     if (e == cudaSuccess && shading) e = upload(&m.shading, shading, size_t(n_tris) * sizeof(ae_triangle));
     if (e != cudaSuccess) {
@@ -598,7 +606,7 @@ ae_rt_status ae_rt_scene_set(ae_rt_ctx* ctx, const ae_bvh_node* tlas, uint32_t n
         table[i].n_nodes = ctx->meshes[i].n_nodes;
         table[i].n_tris = ctx->meshes[i].n_tris;
     }
-    std::vector<ae_bvh_node> flagged = FlagNodes(tlas, n_tlas);
+    const std::vector<PairedNode> paired = DeviceNodes(tlas, n_tlas);
     // object-to-world matrices: the inverse of each instance's world-to-object
     // affine map (the engine's TransformTriangle, surface.hsh:46-61)
     std::vector<float> model(size_t(n_instances) * 12);
@@ -646,7 +654,7 @@ ae_rt_status ae_rt_scene_set(ae_rt_ctx* ctx, const ae_bvh_node* tlas, uint32_t n
         if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
         return e;
     };
-    cudaError_t e = up(reinterpret_cast<void**>(&ctx->d_tlas), flagged.data(), flagged.size() * sizeof(ae_bvh_node));
+    cudaError_t e = up(reinterpret_cast<void**>(&ctx->d_tlas), paired.data(), paired.size() * sizeof(PairedNode));
     if (e == cudaSuccess)
         e = up(reinterpret_cast<void**>(&ctx->d_instances), instances, size_t(n_instances) * sizeof(ae_bvh_instance));
     if (e == cudaSuccess)
@@ -1607,8 +1615,8 @@ __global__ void selftest_shading_kernel(uint32_t kind, const float* in, uint32_t
         const float* r = in + size_t(i) * 14;
         float dist;
         bool nearCull;
-        const bool hit = box_test<false>(r[0], r[1], r[2], r[3], r[4], r[5], 0.0f, 0.0f, 0.0f, r[6], r[7], r[8],
-                                         r[9], r[10], r[11], r[12], r[13], dist, nearCull);
+        const bool hit = box_test(r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], r[10], r[11], r[12],
+                                  r[13], dist, nearCull);
         out[size_t(i) * 2] = hit ? 1.0f : 0.0f;
         out[size_t(i) * 2 + 1] = dist;
         break;

@@ -210,7 +210,7 @@ __device__ __forceinline__ bool in_window(float v) {
 
 __global__ void emit_kernel(const float* verts, const int32_t* material, const float* opacity,
                             const unsigned long long* keys, int n, const int32_t* child, const float* node_box,
-                            const float* leaf_box, ae_bvh_node* nodes, ae_bvh_triangle* tris, uint32_t* order) {
+                            const float* leaf_box, PairedNode* nodes, ae_bvh_triangle* tris, uint32_t* order) {
     const int i = int(blockIdx.x * blockDim.x + threadIdx.x);
     if (i < n - 1) {
         ae_bvh_node nd;
@@ -229,7 +229,7 @@ __global__ void emit_kernel(const float* verts, const int32_t* material, const f
         nd.rightPtr = r;
         nd.padding0 = ok ? 0 : 1;
         nd.padding1 = 0;
-        nodes[i] = nd;
+        nodes[i] = PairNode(nd);
     }
     if (i < n) {
         const uint32_t src = uint32_t(keys[i] & 0xffffffffull);
@@ -328,9 +328,10 @@ extern "C" ae_rt_status ae_rt_mesh_build(ae_rt_ctx* ctx, const float* verts, uin
         ae_bvh_node nd;
         ae_bvh_triangle t[2];
         OneTriangle(v, mat, op, nd, t);
-        BUILD_CUDA(cudaMalloc((void**)&m.nodes, sizeof(ae_bvh_node)));
+        const PairedNode paired = PairNode(nd);
+        BUILD_CUDA(cudaMalloc((void**)&m.nodes, sizeof(PairedNode)));
         cudaError_t e = cudaMalloc((void**)&m.tris, 2 * sizeof(ae_bvh_triangle));
-        if (e == cudaSuccess) e = cudaMemcpy(m.nodes, &nd, sizeof(nd), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(m.nodes, &paired, sizeof(paired), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(m.tris, t, sizeof(t), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             cudaFree(m.nodes);
@@ -418,7 +419,7 @@ extern "C" ae_rt_status ae_rt_mesh_build(ae_rt_ctx* ctx, const float* verts, uin
         else BUILD_CUDA(dalloc((void**)&d_order, size_t(n) * 4));
     }
     emit_kernel<<<blocks, 256, 0, s>>>(d_verts, d_mat, d_op, sorted, int(n), child, node_box, leaf_box,
-                                       reinterpret_cast<ae_bvh_node*>(m.nodes),
+                                       reinterpret_cast<PairedNode*>(m.nodes),
                                        reinterpret_cast<ae_bvh_triangle*>(m.tris), d_order);
     e = cudaGetLastError();
     if (e == cudaSuccess && order_out && !order_dev)
@@ -451,7 +452,21 @@ extern "C" ae_rt_status ae_rt_mesh_get_bvh(ae_rt_ctx* ctx, int32_t mesh_id, ae_b
     if (n_nodes) *n_nodes = m.n_nodes;
     if (n_tris) *n_tris = m.n_tris;
     AE_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (nodes && m.n_nodes) AE_CUDA(ctx, cudaMemcpy(nodes, m.nodes, size_t(m.n_nodes) * 64, cudaMemcpyDefault));
+    if (nodes && m.n_nodes) {
+        // back in the engine's layout (a read-back for inspection and saving,
+        // through host memory whatever the destination)
+        std::vector<PairedNode> paired;
+        std::vector<ae_bvh_node> engine;
+        try {
+            paired.resize(m.n_nodes);
+            engine.resize(m.n_nodes);
+        } catch (...) {
+            return Fail(ctx, AE_RT_OUT_OF_MEMORY, "host memory for the node read-back");
+        }
+        AE_CUDA(ctx, cudaMemcpy(paired.data(), m.nodes, paired.size() * sizeof(PairedNode), cudaMemcpyDeviceToHost));
+        for (size_t i = 0; i < engine.size(); i++) engine[i] = UnpairNode(paired[i]);
+        AE_CUDA(ctx, cudaMemcpy(nodes, engine.data(), engine.size() * sizeof(ae_bvh_node), cudaMemcpyDefault));
+    }
     if (tris && m.n_tris) AE_CUDA(ctx, cudaMemcpy(tris, m.tris, size_t(m.n_tris) * 48, cudaMemcpyDefault));
     return AE_RT_OK;
 }

@@ -24,6 +24,27 @@ struct DeviceMesh {
     uint32_t depth = 0;         // inner-node levels on the longest root-to-leaf path (stack entries it can need)
 };
 
+// A node in the library's device order (load_node in trace_kernels.cuh) from
+// the engine's layout, and back.  padding0 is the node's `slow` word.
+struct PairedNode {
+    uint32_t w[16];
+};
+static_assert(sizeof(PairedNode) == sizeof(ae_bvh_node), "node size");
+
+__host__ __device__ inline PairedNode PairNode(const ae_bvh_node& e) {
+    PairedNode p;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&e);
+    for (int k = 0; k < 16; k++) p.w[k] = src[dev::engine_node_word(k)];
+    return p;
+}
+
+__host__ __device__ inline ae_bvh_node UnpairNode(const PairedNode& p) {
+    ae_bvh_node e;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(&e);
+    for (int k = 0; k < 16; k++) dst[dev::engine_node_word(k)] = p.w[k];
+    return e;
+}
+
 // Grow-only device scratch buffer.
 struct Scratch {
     void* ptr = nullptr;
@@ -59,9 +80,9 @@ struct ae_rt_ctx {
     uint32_t leaf_wait = 0;
     bool count_fetches = false;
     bool near_ties = true;            // complete near-tie detection on closest-hit traces
-    bool staged_rays = false;
+    bool staged_rays = false;         // ray tiles through shared memory by bulk copy
     bool approximate = false;   // AE_RT_CFG_APPROXIMATE
-    uint32_t scene_depth = 0;   // top-level depth + the deepest mesh's: stack entries a scene ray can need         // ray tiles through shared memory by bulk copy
+    uint32_t scene_depth = 0;   // top-level depth + the deepest mesh's: stack entries a scene ray can need
     std::vector<atlas::rt::host::DeviceMesh> meshes;
     // two-level scene: TLAS nodes, instances (TLAS order), mesh table snapshot
     float4* d_tlas = nullptr;

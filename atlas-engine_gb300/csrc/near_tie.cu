@@ -228,15 +228,18 @@ __global__ void retest_kernel(RetestParams p) {
             }
             if (uint32_t(node) >= p.n_nodes) { bad = true; break; }
             const float4* np = p.nodes + size_t(node) * 4;
-            float4 n0, n1, n2, n3;
-            atlas::rt::dev::ldg_node(np, n0, n1, n2, n3);
+            using atlas::rt::dev::lo2;
+            using atlas::rt::dev::hi2;
+            const atlas::rt::dev::NodeBoxes n = atlas::rt::dev::load_node(np);
             // prune by the second distance, and by the window past the nearest
             // beyond which a second distance is not reported
             const double bound = fmin(fmin(p.tmax, second), second_limit(best));
             const float boundf = __double2float_ru(bound);
-            const bool il = box32(of, df, yf, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, tminf, boundf);
-            const bool ir = box32(of, df, yf, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, tminf, boundf);
-            const int32_t l = __float_as_int(n3.x), rr = __float_as_int(n3.y);
+            const bool il = box32(of, df, yf, lo2(n.l_lo_xy), hi2(n.l_lo_xy), lo2(n.l_z), lo2(n.l_hi_xy),
+                                  hi2(n.l_hi_xy), hi2(n.l_z), tminf, boundf);
+            const bool ir = box32(of, df, yf, lo2(n.r_lo_xy), hi2(n.r_lo_xy), lo2(n.r_z), lo2(n.r_hi_xy),
+                                  hi2(n.r_hi_xy), hi2(n.r_z), tminf, boundf);
+            const int32_t l = n.lptr, rr = n.rptr;
             if (il && ir) {
                 if (sp >= kRetestStack) { bad = true; atomicOr(p.error_word, atlas::rt::dev::kErrStackOverflow); break; }
                 stack[sp++] = rr;

@@ -567,8 +567,7 @@ __device__ bool scene_trace_inline(const TraceParams& p, float ox, float oy, flo
     constexpr int kInlineStack = 128;
     int32_t stack[kInlineStack];
     TRay wr{};
-    wr.ox = ox; wr.oy = oy; wr.oz = oz; wr.dx = dx; wr.dy = dy; wr.dz = dz;
-    wr.prepare();
+    wr.set(ox, oy, oz, dx, dy, dz);
     TRay r = wr;
     float hitDist = tmax, hu = 0.0f, hv = 0.0f;
     int32_t hitID = -1, hitInst = -1, curInst = -1;
@@ -595,13 +594,7 @@ __device__ bool scene_trace_inline(const TraceParams& p, float ox, float oy, flo
                     enter = m.n_nodes > 0;
                 }
                 if (enter) {
-                    r.ox = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c0);
-                    r.oy = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c1);
-                    r.oz = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c2);
-                    r.dx = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c0);
-                    r.dy = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c1);
-                    r.dz = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c2);
-                    r.prepare();
+                    r = transform_ray(wr, c0, c1, c2);
                     blasNodes = m.nodes;
                     blasTris = m.tris;
                     node = 0;
@@ -621,7 +614,7 @@ __device__ bool scene_trace_inline(const TraceParams& p, float ox, float oy, flo
                              c = __ldg(blasTris + size_t(tp) * 3 + 2);
                 end = a.w > 0.0f;
                 float t, u, v;
-                const bool hit = tri_test_fast(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, a, b, c, t, u, v);
+                const bool hit = tri_test_fast(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), a, b, c, t, u, v);
                 if (ANY) {
                     if (hit && t > tmin && t < tmax) { occl = true; end = true; }
                 } else if (hit && t > tmin && t < tmax && t < hitDist) {
@@ -634,11 +627,10 @@ __device__ bool scene_trace_inline(const TraceParams& p, float ox, float oy, flo
             node = stack[--sp];
         } else {
             const float4* np = (top ? p.tlas : blasNodes) + size_t(node) * 4;
-            float4 n0, n1, n2, n3;
-            ldg_node(np, n0, n1, n2, n3);
+            const NodeBoxes n = load_node(np);
             bool il, ir, leftFirst;
-            test_children_loose(top ? wr : r, n0, n1, n2, n3, tmin, ANY ? tmax : hitDist, il, ir, leftFirst);
-            const int32_t lptr = __float_as_int(n3.x), rptr = __float_as_int(n3.y);
+            test_children_loose(top ? wr : r, n, tmin, ANY ? tmax : hitDist, il, ir, leftFirst);
+            const int32_t lptr = n.lptr, rptr = n.rptr;
             int32_t next, far;
             if (ANY) {
                 next = il ? lptr : rptr;

@@ -17,8 +17,8 @@
 //  * the traversal stack of each lane lives in shared memory, lane-interleaved
 //    (entry k of lane l at [k][l], conflict-free), with a local-memory spill
 //    area behind it;
-//  * nodes (4 x 16 B) and triangles (3 x 16 B) are fetched with 128-bit
-//    read-only loads;
+//  * nodes are fetched with two 256-bit read-only loads, triangles with three
+//    128-bit ones;
 //  * every ray carries a step cap and a stack bound; exceeding either sets a
 //    flag on the ray and in the context's error word instead of faulting.
 #pragma once
@@ -120,19 +120,91 @@ constexpr int MODE_BATCH = 2;    // many BLASes, one per batch
 
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
 
-// A 64-byte node as two 32-byte read-only loads, one L1 sector each: every lane
-// gathers its own node, so four 16-byte loads would look each sector up twice
-// (the L1 pipeline is the limiter of incoherent rays).  Needs the node at a
-// 32-byte boundary: node arrays are cudaMalloc'ed by the library (256-byte
-// aligned) and 64-byte strided.  Caller-owned arrays (the bounds-checked
-// instance) use ldg4.
-__device__ __forceinline__ void ldg_node(const float4* p, float4& n0, float4& n1, float4& n2, float4& n3) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(n0.x), "=f"(n0.y), "=f"(n0.z), "=f"(n0.w), "=f"(n1.x), "=f"(n1.y), "=f"(n1.z), "=f"(n1.w)
-        : "l"(p));
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8+32];"
-        : "=f"(n2.x), "=f"(n2.y), "=f"(n2.z), "=f"(n2.w), "=f"(n3.x), "=f"(n3.y), "=f"(n3.z), "=f"(n3.w)
-        : "l"(p));
+// Two floats in one 64-bit register pair, and the packed FP32 arithmetic of
+// sm_100 and later on them: one instruction issues the operation for both
+// halves, each rounded to nearest even as the scalar instruction rounds it.
+using f32x2 = unsigned long long;
+
+__host__ __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+#ifdef __CUDA_ARCH__
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+#else
+    return 0;
+#endif
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float(uint32_t(v)); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float(uint32_t(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// A node as the traversal holds it: the two children's boxes in the pairs
+// that the packed slab arithmetic takes, the child pointers, and `slow`, set
+// when a coordinate lies outside the fast-division window (kFastLo / kFastHi).
+struct NodeBoxes {
+    f32x2 l_lo_xy, l_hi_xy, l_z, r_z, r_lo_xy, r_hi_xy;   // *_z: (min z, max z)
+    int32_t lptr, rptr;
+    int32_t slow;
+};
+
+// The library keeps its nodes in device memory in this order (64 bytes, the
+// engine's fields permuted at upload and by the GPU builder):
+//   l.min.xy, l.max.xy, l.min.z, l.max.z, r.min.z, r.max.z |
+//   r.min.xy, r.max.xy, leftPtr, rightPtr, slow, 0
+// so that every pair of coordinates arrives in a register pair without a
+// move: two 32-byte read-only loads, one L1 sector each (four 16-byte loads
+// would look each sector up twice, and the L1 pipeline limits incoherent
+// rays).  Arrays are cudaMalloc'ed by the library, so nodes are 32-byte
+// aligned.
+__device__ __forceinline__ NodeBoxes load_node(const float4* p) {
+    NodeBoxes n;
+    f32x2 ptrs, flags;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(n.l_lo_xy), "=l"(n.l_hi_xy), "=l"(n.l_z), "=l"(n.r_z) : "l"(p));
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4+32];"
+        : "=l"(n.r_lo_xy), "=l"(n.r_hi_xy), "=l"(ptrs), "=l"(flags) : "l"(p));
+    n.lptr = int32_t(uint32_t(ptrs));
+    n.rptr = int32_t(uint32_t(ptrs >> 32));
+    n.slow = int32_t(uint32_t(flags));
+    return n;
+}
+
+// A caller-owned node in the engine's own field order, 16-byte aligned; its
+// coordinates have not been looked at, so it counts as slow.
+__device__ __forceinline__ NodeBoxes load_engine_node(const float4* p) {
+    const float4 n0 = ldg4(p), n1 = ldg4(p + 1), n2 = ldg4(p + 2), n3 = ldg4(p + 3);
+    NodeBoxes n;
+    n.l_lo_xy = pack2(n0.x, n0.y);
+    n.l_hi_xy = pack2(n0.w, n1.x);
+    n.l_z = pack2(n0.z, n1.y);
+    n.r_lo_xy = pack2(n1.z, n1.w);
+    n.r_hi_xy = pack2(n2.y, n2.z);
+    n.r_z = pack2(n2.x, n2.w);
+    n.lptr = __float_as_int(n3.x);
+    n.rptr = __float_as_int(n3.y);
+    n.slow = 1;
+    return n;
+}
+
+// Index in the engine's node (16 words) of word k of the library's.
+__host__ __device__ constexpr int engine_node_word(int k) {
+    // lmin 0-2, lmax 3-5, rmin 6-8, rmax 9-11, pointers 12-13, padding 14-15
+    constexpr int order[16] = { 0, 1, 3, 4, 2, 5, 8, 11, 6, 7, 9, 10, 12, 13, 14, 15 };
+    return order[k];
 }
 
 // IEEE single operations with explicit rounding (no contraction into FMA).
@@ -141,19 +213,21 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 
-// Correctly rounded a / b from y = RN(1/b) without a divide instruction:
-// q0 = RN(a*y) is within 1.5 ulp of a/b; one residual correction
-// q1 = RN(q0 + RN(a - b*q0)*y) makes it faithful; with a faithful quotient the
-// residual a - b*q1 is exact (computed by FMA) and Markstein's theorem
-// (P. Markstein, IBM J. Res. Dev. 34(1), 1990) gives RN(q1 + r1*y) = RN(a/b).
-// Valid while no intermediate under- or overflows, which the callers ensure
-// by range (see kFastLo / kFastHi); everything else takes div.rn.
-__device__ __forceinline__ float div_rn_from_rcp(float a, float b, float y) {
-    float q = __fmul_rn(a, y);
-    float r = __fmaf_rn(-q, b, a);
-    q = __fmaf_rn(r, y, q);
-    r = __fmaf_rn(-q, b, a);
-    return __fmaf_rn(r, y, q);
+// Correctly rounded quotients (c - o) / d of both halves from no = -o,
+// nd = -d and y = RN(1/d), without a divide instruction: q0 = RN(a*y) is
+// within 1.5 ulp of a/d; one residual correction q1 = RN(q0 + RN(a - d*q0)*y)
+// makes it faithful; with a faithful quotient the residual a - d*q1 is exact
+// (computed by FMA) and Markstein's theorem (P. Markstein, IBM J. Res. Dev.
+// 34(1), 1990) gives RN(q1 + r1*y) = RN(a/d).  Valid while no intermediate
+// under- or overflows, which the callers ensure by range (see kFastLo /
+// kFastHi); everything else takes div.rn.
+__device__ __forceinline__ f32x2 slab_quotients(f32x2 c, f32x2 no, f32x2 nd, f32x2 y) {
+    const f32x2 a = add2(c, no);
+    f32x2 q = mul2(a, y);
+    f32x2 r = fma2(q, nd, a);
+    q = fma2(r, y, q);
+    r = fma2(q, nd, a);
+    return fma2(r, y, q);
 }
 
 // Exponent window of the fast quotient: every |origin|, |box coordinate| is 0
@@ -190,35 +264,38 @@ constexpr float kTieWindow = 4e-6f;
 constexpr float kTieWiden = 1.0f + kTieWindow;
 constexpr float kNearMissScale = 9.5367431640625e-07f;   // 2^-20
 
-// IntersectAABB(ray, aabb, tmin, tmax, out dist) -- intersections.hsh:18-34.
-// FAST: quotients through div_rn_from_rcp with (yx, yy, yz) = RN(1/d); the
-// result is bit-identical to the div.rn form.  nearCull: the box was
-// rejected but its entry lies within kTieWindow of the exit bound.
-template <bool FAST>
-__device__ __forceinline__ bool box_test(float ox, float oy, float oz, float dx, float dy, float dz,
-                                         float yx, float yy, float yz,
-                                         float lx, float ly, float lz, float hx, float hy, float hz,
-                                         float tmin, float tmax, float& dist, bool& nearCull) {
-    float t0x, t0y, t0z, t1x, t1y, t1z;
-    if (FAST) {
-        t0x = div_rn_from_rcp(fsub(lx, ox), dx, yx);
-        t0y = div_rn_from_rcp(fsub(ly, oy), dy, yy);
-        t0z = div_rn_from_rcp(fsub(lz, oz), dz, yz);
-        t1x = div_rn_from_rcp(fsub(hx, ox), dx, yx);
-        t1y = div_rn_from_rcp(fsub(hy, oy), dy, yy);
-        t1z = div_rn_from_rcp(fsub(hz, oz), dz, yz);
-    } else {
-        t0x = fdiv(fsub(lx, ox), dx); t0y = fdiv(fsub(ly, oy), dy); t0z = fdiv(fsub(lz, oz), dz);
-        t1x = fdiv(fsub(hx, ox), dx); t1y = fdiv(fsub(hy, oy), dy); t1z = fdiv(fsub(hz, oz), dz);
-    }
-    const float sx = fminf(t0x, t1x), sy = fminf(t0y, t1y), sz = fminf(t0z, t1z);
-    const float bx = fmaxf(t0x, t1x), by = fmaxf(t0y, t1y), bz = fmaxf(t0z, t1z);
-    const float tminf = fmaxf(fmaxf(tmin, sx), fmaxf(sy, sz));
-    const float tmaxf = fminf(fminf(tmax, bx), fminf(by, bz));
+// Three-input minimum / maximum (one instruction; a NaN operand loses).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// IntersectAABB(ray, aabb, tmin, tmax, out dist) -- intersections.hsh:18-34 --
+// from the six slab quotients.  nearCull: the box was rejected but its entry
+// lies within kTieWindow of the exit bound.
+__device__ __forceinline__ bool box_decide(float t0x, float t0y, float t0z, float t1x, float t1y, float t1z,
+                                           float tmin, float tmax, float& dist, bool& nearCull) {
+    const float tminf = fmaxf(tmin, max3(fminf(t0x, t1x), fminf(t0y, t1y), fminf(t0z, t1z)));
+    const float tmaxf = fminf(tmax, min3(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z)));
     const bool hit = tminf <= tmaxf;
     dist = hit ? tminf : tmax;
     nearCull = !hit && tminf <= fmul(tmaxf, kTieWiden);
     return hit;
+}
+
+// The same with the shader's divisions, for any operands.
+__device__ __forceinline__ bool box_test(float ox, float oy, float oz, float dx, float dy, float dz,
+                                         float lx, float ly, float lz, float hx, float hy, float hz,
+                                         float tmin, float tmax, float& dist, bool& nearCull) {
+    return box_decide(fdiv(fsub(lx, ox), dx), fdiv(fsub(ly, oy), dy), fdiv(fsub(lz, oz), dz),
+                      fdiv(fsub(hx, ox), dx), fdiv(fsub(hy, oy), dy), fdiv(fsub(hz, oz), dz), tmin, tmax, dist,
+                      nearCull);
 }
 
 // IntersectTriangle -- intersections.hsh:36-57.  Returns the shader's accept
@@ -360,16 +437,31 @@ struct LaneStack {
     static constexpr uint32_t capacity = SMEM + SPILL;
 };
 
-// One traversal ray in the space of the structure being traversed, with
-// the reciprocals of its direction and the fast-division window flag.
+// One traversal ray in the space of the structure being traversed: its
+// origin and direction, negated, and the correctly rounded reciprocals of the
+// direction, in the pairs (x, y) and (z, z) that the node's coordinate pairs
+// meet, and the fast-division window flag.  Twelve registers, three more than
+// the nine values: the z pair is the price of pairing min z with max z.
 struct TRay {
-    float ox, oy, oz, dx, dy, dz, yx, yy, yz;
+    f32x2 no_xy, no_zz, nd_xy, nd_zz, y_xy, y_zz;
     bool fast;
-    __device__ __forceinline__ void prepare() {
-        yx = __frcp_rn(dx); yy = __frcp_rn(dy); yz = __frcp_rn(dz);
+    __device__ __forceinline__ void set(float ox, float oy, float oz, float dx, float dy, float dz) {
+        const float yz = __frcp_rn(dz);
+        no_xy = pack2(-ox, -oy);
+        no_zz = pack2(-oz, -oz);
+        nd_xy = pack2(-dx, -dy);
+        nd_zz = pack2(-dz, -dz);
+        y_xy = pack2(__frcp_rn(dx), __frcp_rn(dy));
+        y_zz = pack2(yz, yz);
         fast = in_fast_range(ox, true) && in_fast_range(oy, true) && in_fast_range(oz, true) &&
                in_fast_range(dx, false) && in_fast_range(dy, false) && in_fast_range(dz, false);
     }
+    __device__ __forceinline__ float ox() const { return -lo2(no_xy); }
+    __device__ __forceinline__ float oy() const { return -hi2(no_xy); }
+    __device__ __forceinline__ float oz() const { return -lo2(no_zz); }
+    __device__ __forceinline__ float dx() const { return -lo2(nd_xy); }
+    __device__ __forceinline__ float dy() const { return -hi2(nd_xy); }
+    __device__ __forceinline__ float dz() const { return -lo2(nd_zz); }
 };
 
 // Approximate IntersectAABB for the screening below: the six quotients as
@@ -377,12 +469,22 @@ struct TRay {
 // lies within 3 units of 2^-24 (relative) of the shader's quotient and has
 // its sign (zero exactly when c == o), and min / max carry that bound over
 // to the entry lo and exit hi.
-__device__ __forceinline__ void box_approx(const TRay& r, float lx, float ly, float lz, float hx, float hy, float hz,
-                                           float tmin, float tmax, float& lo, float& hi) {
-    const float t0x = fmul(fsub(lx, r.ox), r.yx), t0y = fmul(fsub(ly, r.oy), r.yy), t0z = fmul(fsub(lz, r.oz), r.yz);
-    const float t1x = fmul(fsub(hx, r.ox), r.yx), t1y = fmul(fsub(hy, r.oy), r.yy), t1z = fmul(fsub(hz, r.oz), r.yz);
-    lo = fmaxf(fmaxf(tmin, fminf(t0x, t1x)), fmaxf(fminf(t0y, t1y), fminf(t0z, t1z)));
-    hi = fminf(fminf(tmax, fmaxf(t0x, t1x)), fminf(fmaxf(t0y, t1y), fmaxf(t0z, t1z)));
+__device__ __forceinline__ void box_approx(const TRay& r, f32x2 lo_xy, f32x2 hi_xy, f32x2 z, float tmin, float tmax,
+                                           float& lo, float& hi) {
+    const f32x2 t0 = mul2(add2(lo_xy, r.no_xy), r.y_xy), t1 = mul2(add2(hi_xy, r.no_xy), r.y_xy),
+                tz = mul2(add2(z, r.no_zz), r.y_zz);
+    lo = fmaxf(tmin, max3(fminf(lo2(t0), lo2(t1)), fminf(hi2(t0), hi2(t1)), fminf(lo2(tz), hi2(tz))));
+    hi = fminf(tmax, min3(fmaxf(lo2(t0), lo2(t1)), fmaxf(hi2(t0), hi2(t1)), fmaxf(lo2(tz), hi2(tz))));
+}
+
+// IntersectAABB with the quotients of the fast-division window, bit for bit
+// those of the divisions.
+__device__ __forceinline__ bool box_fast(const TRay& r, f32x2 lo_xy, f32x2 hi_xy, f32x2 z, float tmin, float tmax,
+                                         float& dist, bool& nearCull) {
+    const f32x2 t0 = slab_quotients(lo_xy, r.no_xy, r.nd_xy, r.y_xy),
+                t1 = slab_quotients(hi_xy, r.no_xy, r.nd_xy, r.y_xy),
+                tz = slab_quotients(z, r.no_zz, r.nd_zz, r.y_zz);
+    return box_decide(lo2(t0), hi2(t0), lo2(tz), lo2(t1), hi2(t1), hi2(tz), tmin, tmax, dist, nearCull);
 }
 
 // x <= y decided from approximations x', y' >= 0 that are each within 8 units
@@ -397,26 +499,28 @@ constexpr float kSure = 0.99999904632568359375f;
 // `ordered`), with a missed box reporting the bound as the shader's does;
 // nearCull (only when `ties`): a box was rejected with its entry within
 // kTieWindow of the bound (see kTieWindow).
-// Inside the fast-division window (node.padding0 == 0 marks a node whose
-// coordinates are in it, set by the upload; the ray's own flag; tmin >= 0)
-// the quotients are correctly rounded from the reciprocal (div_rn_from_rcp);
-// outside it and for the BOUNDS variant (whose nodes did not go through the
-// upload) they divide with div.rn.  A traversal that needs only il / ir (any
+// Inside the fast-division window (the node's `slow` word is 0 when its
+// coordinates are in it, set by the upload; the ray's own flag) the quotients
+// are correctly rounded from the reciprocal (slab_quotients); outside it and
+// for the BOUNDS variant (whose nodes did not go through the upload) they
+// divide with div.rn.  The packed form issues 36 instructions for the 12
+// quotients of a node instead of 72; the traversal is bound by instruction
+// issue (72 % of the cycles on 65,536 random triangles), and a million closest
+// hits there went from 1,342 to 1,231 us with it, 400,009 closest hits and as
+// many occlusion tests over 512 instances from 2,312 to 2,084 us.  A traversal that needs only il / ir (any
 // hit: neither ordered nor ties) first screens the boxes with box_approx:
 // every hit decision that the approximations settle with a margin of 16
 // units of 2^-24 is the shader's, and only a lane with a close call (a
 // grazing ray) computes the quotients exactly.  Closest-hit traversals
 // compare entry distances, which are often exactly equal (sibling boxes
 // with a common face), so they take the exact quotients at once.
-template <bool BOUNDS>
-__device__ __forceinline__ void test_children(const TRay& r, const float4& n0, const float4& n1, const float4& n2,
-                                              const float4& n3, float tmin, float bound, bool ordered, bool ties,
-                                              bool& il, bool& ir, bool& leftFirst, bool& nearCull) {
-    const bool fast = !BOUNDS && r.fast && __float_as_int(n3.z) == 0;
+__device__ __forceinline__ void test_children(const TRay& r, const NodeBoxes& n, float tmin, float bound, bool ordered,
+                                              bool ties, bool& il, bool& ir, bool& leftFirst, bool& nearCull) {
+    const bool fast = r.fast && n.slow == 0;
     if (fast && !ordered && !ties && tmin >= 0.0f) {
         float lol, hil, lor, hir;
-        box_approx(r, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, tmin, bound, lol, hil);
-        box_approx(r, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, tmin, bound, lor, hir);
+        box_approx(r, n.l_lo_xy, n.l_hi_xy, n.l_z, tmin, bound, lol, hil);
+        box_approx(r, n.r_lo_xy, n.r_hi_xy, n.r_z, tmin, bound, lor, hir);
         // lo >= tmin >= 0, so a negative exit is a sure miss
         il = hil >= 0.0f && lol <= fmul(hil, kSure);
         ir = hir >= 0.0f && lor <= fmul(hir, kSure);
@@ -429,15 +533,13 @@ __device__ __forceinline__ void test_children(const TRay& r, const float4& n0, c
     bool nl, nr;
     float hl, hr;
     if (fast) {
-        il = box_test<true>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.yx, r.yy, r.yz, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y,
-                            tmin, bound, hl, nl);
-        ir = box_test<true>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.yx, r.yy, r.yz, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w,
-                            tmin, bound, hr, nr);
+        il = box_fast(r, n.l_lo_xy, n.l_hi_xy, n.l_z, tmin, bound, hl, nl);
+        ir = box_fast(r, n.r_lo_xy, n.r_hi_xy, n.r_z, tmin, bound, hr, nr);
     } else {
-        il = box_test<false>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.yx, r.yy, r.yz, n0.x, n0.y, n0.z, n0.w, n1.x,
-                             n1.y, tmin, bound, hl, nl);
-        ir = box_test<false>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.yx, r.yy, r.yz, n1.z, n1.w, n2.x, n2.y, n2.z,
-                             n2.w, tmin, bound, hr, nr);
+        il = box_test(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), lo2(n.l_lo_xy), hi2(n.l_lo_xy), lo2(n.l_z),
+                      lo2(n.l_hi_xy), hi2(n.l_hi_xy), hi2(n.l_z), tmin, bound, hl, nl);
+        ir = box_test(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), lo2(n.r_lo_xy), hi2(n.r_lo_xy), lo2(n.r_z),
+                      lo2(n.r_hi_xy), hi2(n.r_hi_xy), hi2(n.r_z), tmin, bound, hr, nr);
     }
     leftFirst = hl <= hr;
     nearCull = nl || nr;
@@ -452,26 +554,34 @@ __device__ __forceinline__ void test_children(const TRay& r, const float4& n0, c
 // fast-division window it is test_children.
 constexpr float kLoose = 1.00000095367431640625f;   // 1 + 2^-20
 
-__device__ __forceinline__ void test_children_loose(const TRay& r, const float4& n0, const float4& n1,
-                                                    const float4& n2, const float4& n3, float tmin, float bound,
+__device__ __forceinline__ void test_children_loose(const TRay& r, const NodeBoxes& n, float tmin, float bound,
                                                     bool& il, bool& ir, bool& leftFirst) {
-    if (r.fast && __float_as_int(n3.z) == 0 && tmin >= 0.0f) {
+    if (r.fast && n.slow == 0 && tmin >= 0.0f) {
         float lol, hil, lor, hir;
-        box_approx(r, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, tmin, bound, lol, hil);
-        box_approx(r, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, tmin, bound, lor, hir);
+        box_approx(r, n.l_lo_xy, n.l_hi_xy, n.l_z, tmin, bound, lol, hil);
+        box_approx(r, n.r_lo_xy, n.r_hi_xy, n.r_z, tmin, bound, lor, hir);
         il = lol <= fmul(hil, kLoose);
         ir = lor <= fmul(hir, kLoose);
         leftFirst = (il ? lol : bound) <= (ir ? lor : bound);
         return;
     }
     bool unused;
-    test_children<false>(r, n0, n1, n2, n3, tmin, bound, true, false, il, ir, leftFirst, unused);
+    test_children(r, n, tmin, bound, true, false, il, ir, leftFirst, unused);
 }
 
 // vec4(v, w) * inverseMatrix (bvh.hsh:179-180): component i = dot(vec4(v, w),
 // column i), summed left to right with separate roundings.
 __device__ __forceinline__ float xform_row(float x, float y, float z, float w, const float4& c) {
     return fadd(fadd(fadd(fmul(x, c.x), fmul(y, c.y)), fmul(z, c.z)), fmul(w, c.w));
+}
+
+// CheckInstance's object-space ray (bvh.hsh:172-189).
+__device__ __forceinline__ TRay transform_ray(const TRay& w, const float4& c0, const float4& c1, const float4& c2) {
+    const float ox = w.ox(), oy = w.oy(), oz = w.oz(), dx = w.dx(), dy = w.dy(), dz = w.dz();
+    TRay r;
+    r.set(xform_row(ox, oy, oz, 1.0f, c0), xform_row(ox, oy, oz, 1.0f, c1), xform_row(ox, oy, oz, 1.0f, c2),
+          xform_row(dx, dy, dz, 0.0f, c0), xform_row(dx, dy, dz, 0.0f, c1), xform_row(dx, dy, dz, 0.0f, c2));
+    return r;
 }
 
 constexpr uint32_t kTlasInvalid = 0xffffffffu;
@@ -523,6 +633,10 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     static_assert(!LOOSE || (!TIES && !BOUNDS), "loose traversal: no near-tie flag, uploaded nodes");
     static_assert(!CAMERA || (MODE == MODE_MESH && STAGE == 0 && !ANY), "camera rays: single-mesh closest hits");
     __shared__ int32_t s_stack[WARPS][SMEM_STACK][32];
+    // scenes: the world-space ray of each lane while it is inside an instance
+    // (held in registers beside the object-space one it cost spills, and every
+    // step selected between the two)
+    __shared__ uint32_t s_world[TLAS ? WARPS : 1][TLAS ? 10 : 1][32];
     __shared__ __align__(128) float4 s_rays[STAGE > 0 ? WARPS : 1][2][STAGE > 0 ? STAGE * 3 : 1];
     __shared__ __align__(8) uint64_t s_rbar[STAGE > 0 ? WARPS : 1][2];
     const uint32_t lane = threadIdx.x & 31u;
@@ -535,13 +649,12 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     bool live = false;
     bool queueDry = false;          // warp-uniform
     uint32_t rid = 0;
-    TRay wr{};                      // world-space ray (TLAS level)
-    TRay r{};                       // ray in the space of the current BLAS
+    TRay r{};                       // ray in the space of the structure being traversed
     float hitDist = 0, second = 0, hu = 0, hv = 0;
     int32_t hitID = -1, hitInst = -1, curInst = -1;
     int32_t node = 0;
     uint32_t sp = 0, steps = 0, flags = 0, tlasIndex = kTlasInvalid;
-    const float4* blasNodes = p.nodes;
+    const float4* nodes = TLAS ? p.tlas : p.nodes;     // of the structure being traversed
     const float4* blasTris = p.tris;
     bool occl = false;
     bool tieSuspect = false;        // closest hit: a near tie the second distance cannot show (kTieWindow)
@@ -558,18 +671,40 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
 
     // a ray's traversal state from its origin and direction (tmax already set)
     auto beginRay = [&](const float4& o4, const float4& d4, uint32_t nodesHere) {
-        r.ox = o4.x; r.oy = o4.y; r.oz = o4.z;
-        r.dx = d4.x; r.dy = d4.y; r.dz = d4.z;
-        r.prepare();
-        if (TLAS) wr = r;
+        r.set(o4.x, o4.y, o4.z, d4.x, d4.y, d4.z);
+        if (TLAS) {
+            uint32_t* w = &s_world[warp][0][lane];
+            const float v[9] = { lo2(r.no_xy), hi2(r.no_xy), lo2(r.no_zz), lo2(r.nd_xy), hi2(r.nd_xy), lo2(r.nd_zz),
+                                 lo2(r.y_xy), hi2(r.y_xy), lo2(r.y_zz) };
+#pragma unroll
+            for (int k = 0; k < 9; k++) w[k * 32] = __float_as_uint(v[k]);
+            w[9 * 32] = r.fast ? 1u : 0u;
+            nodes = p.tlas;
+        }
         hitDist = tmax; second = tmax; hu = 0.0f; hv = 0.0f;
         hitID = -1; hitInst = -1; curInst = -1;
         node = 0; sp = 0; steps = 0; flags = 0; occl = false; tieSuspect = false;
         tlasIndex = kTlasInvalid;
-        if (MODE == MODE_MESH) { blasNodes = p.nodes; blasTris = p.tris; }
         live = true;
         // NaN direction or an empty BVH: miss (bvh.hsh:204, BVH.cpp:107)
-        if (isnan(r.dx) || isnan(r.dy) || isnan(r.dz) || nodesHere == 0) node = INT32_MIN;
+        if (isnan(d4.x) || isnan(d4.y) || isnan(d4.z) || nodesHere == 0) node = INT32_MIN;
+    };
+
+    // scenes: back to the top level, the world-space ray again
+    auto leaveInstance = [&]() {
+        const uint32_t* w = &s_world[warp][0][lane];
+        float v[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) v[k] = __uint_as_float(w[k * 32]);
+        r.no_xy = pack2(v[0], v[1]);
+        r.no_zz = pack2(v[2], v[2]);
+        r.nd_xy = pack2(v[3], v[4]);
+        r.nd_zz = pack2(v[5], v[5]);
+        r.y_xy = pack2(v[6], v[7]);
+        r.y_zz = pack2(v[8], v[8]);
+        r.fast = w[9 * 32] != 0u;
+        nodes = p.tlas;
+        tlasIndex = kTlasInvalid;
     };
 
     // staged queue of the warp, kept in shared memory between refills (no
@@ -675,7 +810,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                             const BatchDesc& bd = p.batches[find_batch(p.batches, p.n_batches, gi)];
                             ri = gi - bd.first;
                             raySrc = bd.rays;
-                            blasNodes = bd.nodes;
+                            nodes = bd.nodes;
                             blasTris = bd.tris;
                             nodesHere = bd.n_nodes;
                             laneAny = bd.any != 0;
@@ -727,7 +862,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                 }
                 const bool top = TLAS && sp < tlasIndex;
                 if (top) {
-                    tlasIndex = kTlasInvalid;
+                    if (tlasIndex != kTlasInvalid) leaveInstance();
                     if (node < 0) {
                         // CheckInstance: object-space ray, mesh, cull mask
                         const uint32_t ii = uint32_t(~node);
@@ -741,14 +876,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                             enter = m.n_nodes > 0;     // an empty BLAS has no root to visit
                         }
                         if (enter) {
-                            r.ox = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c0);
-                            r.oy = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c1);
-                            r.oz = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c2);
-                            r.dx = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c0);
-                            r.dy = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c1);
-                            r.dz = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c2);
-                            r.prepare();
-                            blasNodes = m.nodes;
+                            r = transform_ray(r, c0, c1, c2);
+                            nodes = m.nodes;
                             blasTris = m.tris;
                             node = 0;
                             tlasIndex = sp;
@@ -759,8 +888,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         continue;
                     }
                 }
-                const float4* nodesArr = top ? p.tlas : blasNodes;
-                const TRay& cr = top ? wr : r;
                 if (BOUNDS && (node < 0 ? uint32_t(~node) >= p.n_tris : uint32_t(node) >= p.n_nodes)) {
                     flags |= kHitFlagOverflow;
                     atomicOr(p.error_word, kErrStackOverflow);
@@ -784,9 +911,10 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         if (COUNT) triCount++;
                         float t, u, v;
                         bool nearMiss = false;
-                        const bool hit = LOOSE ? tri_test_fast(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, a, b, c, t, u, v)
-                                               : tri_test<TIES && !ANY>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, a, b, c, t,
-                                                                        u, v, &nearMiss);
+                        const bool hit = LOOSE ? tri_test_fast(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), a, b, c,
+                                                               t, u, v)
+                                               : tri_test<TIES && !ANY>(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(),
+                                                                        r.dz(), a, b, c, t, u, v, &nearMiss);
                         if (anyQ) {
                             if (hit && t > tmin && t < tmax) { occl = true; end = true; }
                         } else if (hit && t > tmin && t < tmax) {
@@ -806,24 +934,19 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                     if (sp == 0) { done = true; break; }
                     node = st.get(--sp);
                 } else {
-                    const float4* np = nodesArr + size_t(node) * 4;
-                    float4 n0, n1, n2, n3;
-                    if (BOUNDS) {
-                        n0 = ldg4(np); n1 = ldg4(np + 1); n2 = ldg4(np + 2); n3 = ldg4(np + 3);
-                    } else {
-                        ldg_node(np, n0, n1, n2, n3);
-                    }
+                    const float4* np = nodes + size_t(node) * 4;
+                    const NodeBoxes n = BOUNDS ? load_engine_node(np) : load_node(np);
                     if (COUNT) nodeCount++;
-                    const int32_t lptr = __float_as_int(n3.x), rptr = __float_as_int(n3.y);
+                    const int32_t lptr = n.lptr, rptr = n.rptr;
                     bool il, ir, leftFirst, nearCull = false;
                     if (LOOSE)
-                        test_children_loose(cr, n0, n1, n2, n3, tmin, anyQ ? tmax : hitDist, il, ir, leftFirst);
+                        test_children_loose(r, n, tmin, anyQ ? tmax : hitDist, il, ir, leftFirst);
                     else
                         // the batched launch decides the query kind per lane at run time; with
                         // both box tests compiled into it, it ran 8 % slower (11.85 against
                         // 10.99 ms on 64 meshes), so every lane takes the exact test there
-                        test_children<BOUNDS>(cr, n0, n1, n2, n3, tmin, anyQ ? tmax : hitDist, BATCH || !anyQ,
-                                              TIES && !anyQ, il, ir, leftFirst, nearCull);
+                        test_children(r, n, tmin, anyQ ? tmax : hitDist, BATCH || !anyQ, TIES && !anyQ, il, ir,
+                                      leftFirst, nearCull);
                     if (TIES && !anyQ) tieSuspect = tieSuspect || nearCull;
                     int32_t next, far;
                     if (anyQ) {

@@ -61,13 +61,11 @@ __device__ __forceinline__ float shading_opacity(const TransParams& p, float4 d0
 template <bool ANY>
 __global__ void transparency_kernel(TransParams p) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
-    const uint32_t n = p.count ? min(*p.count, p.n) : p.n;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint32_t nRays = p.count ? min(*p.count, p.n) : p.n;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nRays; i += stride) {
         const float4 o4 = p.rays[i * 3], d4 = p.rays[i * 3 + 1];
         TRay wr{};
-        wr.ox = o4.x; wr.oy = o4.y; wr.oz = o4.z;
-        wr.dx = d4.x; wr.dy = d4.y; wr.dz = d4.z;
-        wr.prepare();
+        wr.set(o4.x, o4.y, o4.z, d4.x, d4.y, d4.z);
         TRay r = wr;
         const float tMin = p.tmin, tMax = p.per_ray_tmax ? p.rays[i * 3 + 2].x : p.tmax;
         float hitDist = tMax, hu = 0.0f, hv = 0.0f, transparency = 1.0f;
@@ -100,13 +98,7 @@ __global__ void transparency_kernel(TransParams p) {
                         curInst = int32_t(ii);
                         const MeshDesc m = p.meshes[__float_as_int(c3.x)];
                         matOffset = __float_as_int(c3.y);
-                        r.ox = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c0);
-                        r.oy = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c1);
-                        r.oz = xform_row(wr.ox, wr.oy, wr.oz, 1.0f, c2);
-                        r.dx = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c0);
-                        r.dy = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c1);
-                        r.dz = xform_row(wr.dx, wr.dy, wr.dz, 0.0f, c2);
-                        r.prepare();
+                        r = transform_ray(wr, c0, c1, c2);
                         blasNodes = m.nodes;
                         shading = m.shading;
                         if ((__float_as_uint(c3.w) & p.cull_mask) != 0u && m.n_nodes > 0 && shading) {
@@ -117,12 +109,11 @@ __global__ void transparency_kernel(TransParams p) {
                         pop = true;
                     } else {
                         const float4* np = p.tlas + size_t(nodePtr) * 4;
-                        const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
+                        const NodeBoxes n = load_node(np);
                         bool il, ir, leftFirst;
                         bool nearCullUnused;   // near-tie detection is the closest-hit trace's alone
-                        test_children<false>(r, n0, n1, n2, n3, tMin, ANY ? tMax : hitDist, !ANY, false, il, ir,
-                                             leftFirst, nearCullUnused);
-                        const int32_t l = __float_as_int(n3.x), rr = __float_as_int(n3.y);
+                        test_children(r, n, tMin, ANY ? tMax : hitDist, !ANY, false, il, ir, leftFirst, nearCullUnused);
+                        const int32_t l = n.lptr, rr = n.rptr;
                         if (ANY) {
                             next = il ? l : rr;
                             if (il && ir) {
@@ -148,7 +139,7 @@ __global__ void transparency_kernel(TransParams p) {
                         const float4 d0 = __ldg(sp4 + 3), d1 = __ldg(sp4 + 4), d2 = __ldg(sp4 + 5);
                         end = d1.z > 0.0f;
                         float t, u, v;
-                        const bool hit = tri_test(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, a, b, c, t, u, v);
+                        const bool hit = tri_test(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), a, b, c, t, u, v);
                         if (ANY) {
                             if (hit && t > tMin && t < tMax)
                                 leaf = __fmul_rn(leaf, __fsub_rn(1.0f, shading_opacity(p, d0, d2, matOffset, u, v)));
@@ -164,12 +155,11 @@ __global__ void transparency_kernel(TransParams p) {
                     pop = true;
                 } else {
                     const float4* np = blasNodes + size_t(nodePtr) * 4;
-                    const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
+                    const NodeBoxes n = load_node(np);
                     bool il, ir, leftFirst;
                     bool nearCullUnused;   // near-tie detection is the closest-hit trace's alone
-                    test_children<false>(r, n0, n1, n2, n3, tMin, ANY ? tMax : hitDist, !ANY, false, il, ir, leftFirst,
-                                         nearCullUnused);
-                    const int32_t l = __float_as_int(n3.x), rr = __float_as_int(n3.y);
+                    test_children(r, n, tMin, ANY ? tMax : hitDist, !ANY, false, il, ir, leftFirst, nearCullUnused);
+                    const int32_t l = n.lptr, rr = n.rptr;
                     if (ANY) {
                         next = il ? l : rr;
                         if (il && ir) {
