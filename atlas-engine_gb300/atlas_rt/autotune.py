@@ -6,10 +6,6 @@ Searches, for one workload on the current GPU, the axes
     (64, 32), (256, 16), (128, 16));
   * refill_steps: traversal steps a warp takes between two queue refills,
     i.e. the size of the per-warp ray tile (8 ... 64);
-  * refill_below: refill as soon as fewer lanes than this still traverse
-    (never, 8, 16, 24);
-  * leaf_wait: closest-hit lanes at a leaf wait for this many leaf lanes
-    (0, 2, 4, 6);
   * workload-specific axes (for the path tracer: the number of image tiles,
     which sets the size of its wavefront queues);
 by coordinate descent: starting from the library's defaults, each axis in
@@ -26,11 +22,9 @@ from pathlib import Path
 SHAPES = [(128, 32), (64, 32), (256, 16), (128, 16)]
 AXES = {
     "shape": SHAPES,
-    "refill_steps": [8, 16, 32, 64],
-    "refill_below": [33, 8, 16, 24],      # 33: never refill early
-    "leaf_wait": [0, 2, 4, 6],
+    "refill_steps": [8, 16, 24, 32, 64],
 }
-DEFAULTS = {"shape": (128, 32), "refill_steps": 32, "refill_below": 8, "leaf_wait": 0}
+DEFAULTS = {"shape": (128, 32), "refill_steps": 24}
 CONFIG_KEYS = ("threads_per_block", "stack_entries_smem", "refill_steps", "refill_below", "leaf_wait",
                "blocks_per_sm")
 

@@ -44,14 +44,19 @@ using atlas::rt::dev::MODE_MESH;
 using atlas::rt::dev::MODE_SCENE;
 
 template <bool ANY, bool COUNT, int MODE, int W, int S, bool TIES = true, int STAGE = 0, bool LOOSE = false,
-          bool DEEP = false, bool CAMERA = false>
+          int STACK = kStackEntries, bool CAMERA = false>
 void* KernelFor() {
-    // single-mesh kernels keep <= 64 registers; scene / batched kernels carry
-    // more per-lane state and get ~73
-    constexpr int minBlocks = MODE == MODE_MESH ? 32 / W : (28 / W > 0 ? 28 / W : 1);
+    // 64 registers for 32 warps an SM; the scene kernels that detect near ties
+    // and the batched ones carry more per-lane state and get 72 (at 64: 1,892
+    // against 1,842 us for the 512-instance scene, 3,046 against 3,003 us for
+    // 64 meshes; the scene kernels without ties gain, a path-traced sample
+    // 1,378 against 1,410 us).  36 or 40 warps of single-mesh kernels lose to
+    // spills (1,126 against 1,074 us for a million random closest hits).
+    constexpr bool wide = MODE == MODE_BATCH || (MODE == MODE_SCENE && TIES && !ANY);
+    constexpr int minBlocks = wide ? (28 / W > 0 ? 28 / W : 1) : 32 / W;
     return reinterpret_cast<void*>(
-        &atlas::rt::dev::trace_kernel<ANY, COUNT, MODE, W, S, (DEEP ? kDeepStackEntries : kStackEntries) - S,
-                                      minBlocks, false, TIES && !ANY, STAGE, LOOSE, CAMERA>);
+        &atlas::rt::dev::trace_kernel<ANY, COUNT, MODE, W, S, STACK - S, minBlocks, false, TIES && !ANY, STAGE, LOOSE,
+                                      CAMERA>);
 }
 
 // ties = false: the caller discards the near-tie flag (the library's path
@@ -61,18 +66,21 @@ void* KernelFor() {
 // (AE_RT_CFG_STAGED_RAYS; single-mesh and scene launches without counters).
 // loose: the approximate traversal (AE_RT_CFG_APPROXIMATE): single-mesh and
 // scene launches without counters or staged rays, no near-tie flag.
-template <int W, int S>
+// STACK: stack entries per lane; S of them when no tree of the launch can
+// need more (no local memory), else kStackEntries.  Counting and staged
+// launches always hold kStackEntries.
+template <int W, int S, int STACK>
 void* PickShape(bool any, bool count, int mode, bool ties, bool staged, bool loose, bool camera) {
     constexpr int T = atlas::rt::dev::kStageRays;
     if (camera)
-        return ties ? KernelFor<false, false, MODE_MESH, W, S, true, 0, false, false, true>()
-                    : KernelFor<false, false, MODE_MESH, W, S, false, 0, false, false, true>();
+        return ties ? KernelFor<false, false, MODE_MESH, W, S, true, 0, false, STACK, true>()
+                    : KernelFor<false, false, MODE_MESH, W, S, false, 0, false, STACK, true>();
     if (loose && mode == MODE_SCENE && !count && !staged)
-        return any ? KernelFor<true, false, MODE_SCENE, W, S, false, 0, true>()
-                   : KernelFor<false, false, MODE_SCENE, W, S, false, 0, true>();
+        return any ? KernelFor<true, false, MODE_SCENE, W, S, false, 0, true, STACK>()
+                   : KernelFor<false, false, MODE_SCENE, W, S, false, 0, true, STACK>();
     if (loose && mode == MODE_MESH && !count && !staged)
-        return any ? KernelFor<true, false, MODE_MESH, W, S, false, 0, true>()
-                   : KernelFor<false, false, MODE_MESH, W, S, false, 0, true>();
+        return any ? KernelFor<true, false, MODE_MESH, W, S, false, 0, true, STACK>()
+                   : KernelFor<false, false, MODE_MESH, W, S, false, 0, true, STACK>();
     if (staged && !count && mode != MODE_BATCH) {
         if (mode == MODE_SCENE) {
             if (any) return KernelFor<true, false, MODE_SCENE, W, S, true, T>();
@@ -84,20 +92,24 @@ void* PickShape(bool any, bool count, int mode, bool ties, bool staged, bool loo
                     : KernelFor<false, false, MODE_MESH, W, S, false, T>();
     }
     if (mode == MODE_BATCH) {
-        if (!ties)
-            return count ? KernelFor<false, true, MODE_BATCH, W, S, false>() : KernelFor<false, false, MODE_BATCH, W, S, false>();
-        return count ? KernelFor<false, true, MODE_BATCH, W, S>() : KernelFor<false, false, MODE_BATCH, W, S>();
+        if (count) return ties ? KernelFor<false, true, MODE_BATCH, W, S>() : KernelFor<false, true, MODE_BATCH, W, S, false>();
+        return ties ? KernelFor<false, false, MODE_BATCH, W, S, true, 0, false, STACK>()
+                    : KernelFor<false, false, MODE_BATCH, W, S, false, 0, false, STACK>();
     }
     if (mode == MODE_SCENE) {
-        if (any) return count ? KernelFor<true, true, MODE_SCENE, W, S>() : KernelFor<true, false, MODE_SCENE, W, S>();
-        if (!ties)
-            return count ? KernelFor<false, true, MODE_SCENE, W, S, false>() : KernelFor<false, false, MODE_SCENE, W, S, false>();
-        return count ? KernelFor<false, true, MODE_SCENE, W, S>() : KernelFor<false, false, MODE_SCENE, W, S>();
+        if (count)
+            return any ? KernelFor<true, true, MODE_SCENE, W, S>()
+                       : ties ? KernelFor<false, true, MODE_SCENE, W, S>() : KernelFor<false, true, MODE_SCENE, W, S, false>();
+        if (any) return KernelFor<true, false, MODE_SCENE, W, S, true, 0, false, STACK>();
+        return ties ? KernelFor<false, false, MODE_SCENE, W, S, true, 0, false, STACK>()
+                    : KernelFor<false, false, MODE_SCENE, W, S, false, 0, false, STACK>();
     }
-    if (any) return count ? KernelFor<true, true, MODE_MESH, W, S>() : KernelFor<true, false, MODE_MESH, W, S>();
-    if (!ties)
-        return count ? KernelFor<false, true, MODE_MESH, W, S, false>() : KernelFor<false, false, MODE_MESH, W, S, false>();
-    return count ? KernelFor<false, true, MODE_MESH, W, S>() : KernelFor<false, false, MODE_MESH, W, S>();
+    if (count)
+        return any ? KernelFor<true, true, MODE_MESH, W, S>()
+                   : ties ? KernelFor<false, true, MODE_MESH, W, S>() : KernelFor<false, true, MODE_MESH, W, S, false>();
+    if (any) return KernelFor<true, false, MODE_MESH, W, S, true, 0, false, STACK>();
+    return ties ? KernelFor<false, false, MODE_MESH, W, S, true, 0, false, STACK>()
+                : KernelFor<false, false, MODE_MESH, W, S, false, 0, false, STACK>();
 }
 
 // The deep variants (kDeepStackEntries, exact traversal, the default shape)
@@ -105,22 +117,27 @@ void* PickShape(bool any, bool count, int mode, bool ties, bool staged, bool loo
 // kStackEntries entries.
 void* PickDeep(bool any, int mode, bool ties) {
     if (mode == MODE_SCENE) {
-        if (any) return KernelFor<true, false, MODE_SCENE, 4, 32, true, 0, false, true>();
-        return ties ? KernelFor<false, false, MODE_SCENE, 4, 32, true, 0, false, true>()
-                    : KernelFor<false, false, MODE_SCENE, 4, 32, false, 0, false, true>();
+        if (any) return KernelFor<true, false, MODE_SCENE, 4, 32, true, 0, false, kDeepStackEntries>();
+        return ties ? KernelFor<false, false, MODE_SCENE, 4, 32, true, 0, false, kDeepStackEntries>()
+                    : KernelFor<false, false, MODE_SCENE, 4, 32, false, 0, false, kDeepStackEntries>();
     }
-    if (any) return KernelFor<true, false, MODE_MESH, 4, 32, true, 0, false, true>();
-    return ties ? KernelFor<false, false, MODE_MESH, 4, 32, true, 0, false, true>()
-                : KernelFor<false, false, MODE_MESH, 4, 32, false, 0, false, true>();
+    if (any) return KernelFor<true, false, MODE_MESH, 4, 32, true, 0, false, kDeepStackEntries>();
+    return ties ? KernelFor<false, false, MODE_MESH, 4, 32, true, 0, false, kDeepStackEntries>()
+                : KernelFor<false, false, MODE_MESH, 4, 32, false, 0, false, kDeepStackEntries>();
 }
 
-void* PickKernelShape(int shape, bool any, bool count, int mode, bool ties = true, bool staged = false,
+// depth: the stack entries that the launch's trees can need (at most
+// kStackEntries).
+void* PickKernelShape(int shape, uint32_t depth, bool any, bool count, int mode, bool ties = true, bool staged = false,
                       bool loose = false, bool camera = false) {
+    const bool shallow = depth < uint32_t(kShapes[shape].smem);    // one entry marks the end
     switch (shape) {
-    case 1: return PickShape<2, 32>(any, count, mode, ties, staged, loose, camera);
-    case 2: return PickShape<8, 16>(any, count, mode, ties, staged, loose, camera);
-    case 3: return PickShape<4, 16>(any, count, mode, ties, staged, loose, camera);
-    default: return PickShape<4, 32>(any, count, mode, ties, staged, loose, camera);
+    case 1: return shallow ? PickShape<2, 32, 32>(any, count, mode, ties, staged, loose, camera)
+                           : PickShape<2, 32, kStackEntries>(any, count, mode, ties, staged, loose, camera);
+    case 2: return PickShape<8, 16, kStackEntries>(any, count, mode, ties, staged, loose, camera);
+    case 3: return PickShape<4, 16, kStackEntries>(any, count, mode, ties, staged, loose, camera);
+    default: return shallow ? PickShape<4, 32, 32>(any, count, mode, ties, staged, loose, camera)
+                            : PickShape<4, 32, kStackEntries>(any, count, mode, ties, staged, loose, camera);
     }
 }
 
@@ -236,21 +253,19 @@ uint32_t* WorkCounter(ae_rt_ctx* ctx) {
     return ctx->d_counter + (k == 0 ? 0u : k + 1u);          // word 1 is the error word
 }
 
-// depth: stack entries the launch's tree can need (0: the batched launch,
-// whose meshes keep to kStackEntries or report overflow).
+// depth: stack entries the launch's trees can need (batched launches hold
+// kStackEntries at most and report overflow beyond).
 // camera: the rays are p.cam's camera rays (single mesh, closest hit, a tree
 // within kStackEntries, exact, no counters: Trace checks this).
-ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStream_t s, bool ties = true,
-                    uint32_t depth = 0, bool camera = false) {
+ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStream_t s, bool ties, uint32_t depth,
+                    bool camera = false) {
     if (p.work_counter == ctx->d_counter) p.work_counter = WorkCounter(ctx);
     AE_CUDA(ctx, cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
-    p.refill_below = ctx->refill_below;
-    p.leaf_wait = ctx->leaf_wait;
     const bool deep = depth > uint32_t(kStackEntries) && mode != MODE_BATCH;
     void* fn = deep ? PickDeep(any, mode, ties && ctx->near_ties)
-                    : PickKernelShape(ctx->shape, any, ctx->count_fetches, mode, ties && ctx->near_ties,
+                    : PickKernelShape(ctx->shape, depth, any, ctx->count_fetches, mode, ties && ctx->near_ties,
                                       ctx->staged_rays, ctx->approximate, camera);
     const uint32_t threads = deep ? 128u : ctx->threads;
     const uint32_t grid = GridFor(ctx, fn, p.n_rays, threads);
@@ -457,10 +472,9 @@ ae_rt_status ae_rt_ctx_create(const ae_rt_config* cfg, ae_rt_ctx** out) {
     ctx->near_ties = (c.flags & AE_RT_CFG_NO_NEAR_TIES) == 0;
     ctx->staged_rays = (c.flags & AE_RT_CFG_STAGED_RAYS) != 0;
     ctx->approximate = (c.flags & AE_RT_CFG_APPROXIMATE) != 0;
-    ctx->refill_steps = c.refill_steps;
-    ctx->refill_below = c.refill_below == 0 ? atlas::rt::dev::kDefaultRefillBelow
-                                            : (c.refill_below > 32 ? 0u : c.refill_below);
-    ctx->leaf_wait = c.leaf_wait > 32 ? 32u : c.leaf_wait;
+    ctx->refill_steps = c.refill_steps ? c.refill_steps : atlas::rt::dev::kDefaultRefillSteps;
+    // refills that should not wait for a full burst: short bursts
+    if (c.refill_below > 0 && c.refill_below <= 32) ctx->refill_steps = std::min(ctx->refill_steps, 8u);
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, 8 * sizeof(uint32_t));
@@ -737,9 +751,11 @@ struct ae_rt_batch_plan {
 
 namespace {
 
-// Device batch table for a launch; returns the total ray count.
+// Device batch table for a launch, its total ray count and the depth of its
+// deepest tree.
 ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32_t n,
-                            std::vector<atlas::rt::dev::BatchDesc>& table, uint32_t& total) {
+                            std::vector<atlas::rt::dev::BatchDesc>& table, uint32_t& total, uint32_t& depth) {
+    depth = 0;
     table.resize(n);
     uint64_t first = 0;
     for (uint32_t i = 0; i < n; i++) {
@@ -750,6 +766,7 @@ ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32
             return Fail(ctx, AE_RT_INVALID_ARG, "batch " + std::to_string(i) + ": batched traces take device buffers");
         const DeviceMesh& m = ctx->meshes[size_t(b.mesh_id)];
         atlas::rt::dev::BatchDesc& d = table[i];
+        depth = std::max(depth, m.depth);
         d.nodes = m.nodes;
         d.tris = m.tris;
         d.rays = reinterpret_cast<const float4*>(b.rays);
@@ -779,8 +796,6 @@ TraceParams BatchParams(ae_rt_ctx* ctx, const atlas::rt::dev::BatchDesc* d_batch
     p.batches = d_batches;
     p.n_batches = n;
     p.refill_steps = ctx->refill_steps;
-    p.refill_below = ctx->refill_below;
-    p.leaf_wait = ctx->leaf_wait;
     p.max_steps = 0xffffffffu;
     return p;
 }
@@ -793,8 +808,8 @@ ae_rt_status ae_rt_trace_batched(ae_rt_ctx* ctx, const ae_batch_desc* batches, u
     if (!batches) return Fail(ctx, AE_RT_INVALID_ARG, "null batch table");
     AE_CUDA(ctx, cudaSetDevice(ctx->device));
     std::vector<atlas::rt::dev::BatchDesc> table;
-    uint32_t total = 0;
-    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total);
+    uint32_t total = 0, depth = 0;
+    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total, depth);
     if (st != AE_RT_OK) return st;
     if (total == 0) return AE_RT_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -803,7 +818,7 @@ ae_rt_status ae_rt_trace_batched(ae_rt_ctx* ctx, const ae_batch_desc* batches, u
                                  cudaMemcpyHostToDevice, s));
     TraceParams p = BatchParams(ctx, static_cast<atlas::rt::dev::BatchDesc*>(ctx->batch_table.ptr), n_batches,
                                 total, ctx->d_counter);
-    return Launch(ctx, false, MODE_BATCH, p, s);
+    return Launch(ctx, false, MODE_BATCH, p, s, true, depth);
 }
 
 ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32_t n_batches,
@@ -813,8 +828,8 @@ ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batche
     if (n_batches == 0 || !batches) return Fail(ctx, AE_RT_INVALID_ARG, "a plan needs at least one batch");
     AE_CUDA(ctx, cudaSetDevice(ctx->device));
     std::vector<atlas::rt::dev::BatchDesc> table;
-    uint32_t total = 0;
-    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total);
+    uint32_t total = 0, depth = 0;
+    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total, depth);
     if (st != AE_RT_OK) return st;
     auto* plan = new (std::nothrow) ae_rt_batch_plan;
     if (!plan) return AE_RT_OUT_OF_MEMORY;
@@ -832,7 +847,7 @@ ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batche
         TraceParams p = BatchParams(ctx, plan->d_batches, n_batches, total, plan->d_counter);
         cudaError_t le = cudaMemsetAsync(plan->d_counter, 0, sizeof(uint32_t), cap);
         void* args[] = { &p };
-        void* fn = PickKernelShape(ctx->shape, false, false, MODE_BATCH, ctx->near_ties);
+        void* fn = PickKernelShape(ctx->shape, depth, false, false, MODE_BATCH, ctx->near_ties);
         if (le == cudaSuccess)
             le = cudaLaunchKernel(fn, dim3(GridFor(ctx, fn, total)), dim3(ctx->threads), args, 0, cap);
         e = cudaStreamEndCapture(cap, &plan->graph);

@@ -76,8 +76,6 @@ struct ae_rt_ctx {
     uint32_t threads = 128;
     uint32_t max_steps_cfg = 0;
     uint32_t refill_steps = 0;
-    uint32_t refill_below = 0;
-    uint32_t leaf_wait = 0;
     bool count_fetches = false;
     bool near_ties = true;            // complete near-tie detection on closest-hit traces
     bool staged_rays = false;         // ray tiles through shared memory by bulk copy

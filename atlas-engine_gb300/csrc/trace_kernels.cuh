@@ -77,9 +77,7 @@ struct TraceParams {
     const struct BatchDesc* batches;
     uint32_t n_batches;
     uint32_t refill_steps;       // traversal steps between warp refills
-    uint32_t refill_below;       // refill early when fewer lanes than this still traverse (0: never)
     uint32_t per_ray_tmax;       // nonzero: a ray's tmax is its PackedRay hit.x (shadow queues)
-    uint32_t leaf_wait;          // closest hit: a lane at a leaf waits for this many leaf lanes (0: never)
     CameraParams cam;            // the camera variant: ray i is camera_ray(cam, i), `rays` unused
 };
 
@@ -109,10 +107,8 @@ __host__ __device__ constexpr uint32_t default_step_cap(uint32_t n_nodes) {
     return 4ull * n_nodes + 64ull > 0xffffffffull ? 0xffffffffu : uint32_t(4ull * n_nodes + 64ull);
 }
 
-// ae_rt_config::refill_below when left 0 (lanes; 0 = never refill early):
-// measured best with a 32-step burst on the terrain + boxes camera pass
-// (0.913 against 0.974 ms for 64 steps and no early refill).
-constexpr uint32_t kDefaultRefillBelow = 8;
+// ae_rt_config::refill_steps when left 0.
+constexpr uint32_t kDefaultRefillSteps = 24;
 
 constexpr int MODE_MESH = 0;     // one BLAS
 constexpr int MODE_SCENE = 1;    // TLAS over instances
@@ -152,6 +148,10 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     return r;
 }
 
+// The node value that ends a traversal: the bottom of the stack, and no
+// pointer of a valid tree (arrays hold fewer than 2^31 - 1 elements).
+constexpr int32_t kStackEnd = INT32_MIN;
+
 // A node as the traversal holds it: the two children's boxes in the pairs
 // that the packed slab arithmetic takes, the child pointers, and `slow`, set
 // when a coordinate lies outside the fast-division window (kFastLo / kFastHi).
@@ -184,7 +184,8 @@ __device__ __forceinline__ NodeBoxes load_node(const float4* p) {
 }
 
 // A caller-owned node in the engine's own field order, 16-byte aligned; its
-// coordinates have not been looked at, so it counts as slow.
+// coordinates have not been looked at, so it counts as slow.  A pointer equal
+// to kStackEnd becomes its neighbour, which is past any triangle array too.
 __device__ __forceinline__ NodeBoxes load_engine_node(const float4* p) {
     const float4 n0 = ldg4(p), n1 = ldg4(p + 1), n2 = ldg4(p + 2), n3 = ldg4(p + 3);
     NodeBoxes n;
@@ -194,8 +195,8 @@ __device__ __forceinline__ NodeBoxes load_engine_node(const float4* p) {
     n.r_lo_xy = pack2(n1.z, n1.w);
     n.r_hi_xy = pack2(n2.y, n2.z);
     n.r_z = pack2(n2.x, n2.w);
-    n.lptr = __float_as_int(n3.x);
-    n.rptr = __float_as_int(n3.y);
+    n.lptr = max(__float_as_int(n3.x), kStackEnd + 1);
+    n.rptr = max(__float_as_int(n3.y), kStackEnd + 1);
     n.slow = 1;
     return n;
 }
@@ -307,22 +308,26 @@ __device__ __forceinline__ bool box_test(float ox, float oy, float oz, float dx,
 // m = 2^-20 Sd (S0+S1) (Ss+S0+S1) (2^-20 = 16 ulps of 1).  The tests are
 // taken multiplied by |den| (u |den| + m >= 0, ...), one correctly rounded
 // FMA each, so the oracle reproduces them.  slack (optional) receives |den| and m.
-template <bool NEAR = false>
-__device__ __forceinline__ bool tri_test(float ox, float oy, float oz, float dx, float dy, float dz,
-                                         const float4& a, const float4& b, const float4& c,
-                                         float& t, float& u, float& v, bool* nearMiss = nullptr,
-                                         float* slack = nullptr) {
+struct TriTerms {
+    float den, nt, nu, nv;     // t = nt / den, u = nu / den, v = nv / den
+    float m;                   // the slack (NEAR)
+};
+
+template <bool NEAR>
+__device__ __forceinline__ TriTerms tri_terms(float ox, float oy, float oz, float dx, float dy, float dz,
+                                              const float4& a, const float4& b, const float4& c) {
+    TriTerms r;
     const float e0x = fsub(b.x, a.x), e0y = fsub(b.y, a.y), e0z = fsub(b.z, a.z);
     const float e1x = fsub(c.x, a.x), e1y = fsub(c.y, a.y), e1z = fsub(c.z, a.z);
     const float sx = fsub(ox, a.x), sy = fsub(oy, a.y), sz = fsub(oz, a.z);
     // the slack's scale, folded at once so that one value stays live
-    float m = 0.0f;
+    r.m = 0.0f;
     if (NEAR) {
         const float s01 = fadd(fadd(fadd(fabsf(e0x), fabsf(e0y)), fabsf(e0z)),
                                fadd(fadd(fabsf(e1x), fabsf(e1y)), fabsf(e1z)));
         const float ss = fadd(fadd(fabsf(sx), fabsf(sy)), fabsf(sz));
         const float sd = fadd(fadd(fabsf(dx), fabsf(dy)), fabsf(dz));
-        m = fmul(fmul(fmul(sd, s01), fadd(ss, s01)), kNearMissScale);
+        r.m = fmul(fmul(fmul(sd, s01), fadd(ss, s01)), kNearMissScale);
     }
     // p = cross(s, e0), q = cross(d, e1)
     const float px = fsub(fmul(sy, e0z), fmul(e0y, sz));
@@ -331,17 +336,58 @@ __device__ __forceinline__ bool tri_test(float ox, float oy, float oz, float dx,
     const float qx = fsub(fmul(dy, e1z), fmul(e1y, dz));
     const float qy = fsub(fmul(dz, e1x), fmul(e1z, dx));
     const float qz = fsub(fmul(dx, e1y), fmul(e1x, dy));
-    const float den = fadd(fadd(fmul(qx, e0x), fmul(qy, e0y)), fmul(qz, e0z));
-    t = fdiv(fadd(fadd(fmul(px, e1x), fmul(py, e1y)), fmul(pz, e1z)), den);
-    u = fdiv(fadd(fadd(fmul(qx, sx), fmul(qy, sy)), fmul(qz, sz)), den);
-    v = fdiv(fadd(fadd(fmul(px, dx), fmul(py, dy)), fmul(pz, dz)), den);
+    r.den = fadd(fadd(fmul(qx, e0x), fmul(qy, e0y)), fmul(qz, e0z));
+    r.nt = fadd(fadd(fmul(px, e1x), fmul(py, e1y)), fmul(pz, e1z));
+    r.nu = fadd(fadd(fmul(qx, sx), fmul(qy, sy)), fmul(qz, sz));
+    r.nv = fadd(fadd(fmul(px, dx), fmul(py, dy)), fmul(pz, dz));
+    return r;
+}
+
+template <bool NEAR>
+__device__ __forceinline__ bool tri_decide(const TriTerms& r, float& t, float& u, float& v, bool* nearMiss) {
+    t = fdiv(r.nt, r.den);
+    u = fdiv(r.nu, r.den);
+    v = fdiv(r.nv, r.den);
     if (NEAR) {
-        const float ad = fabsf(den);
-        *nearMiss = __fmaf_rn(u, ad, m) >= 0.0f && __fmaf_rn(v, ad, m) >= 0.0f &&
-                    __fmaf_rn(fsub(1.0f, fadd(u, v)), ad, fadd(m, m)) >= 0.0f;
-        if (slack) { slack[0] = ad; slack[1] = m; }
+        const float ad = fabsf(r.den);
+        *nearMiss = __fmaf_rn(u, ad, r.m) >= 0.0f && __fmaf_rn(v, ad, r.m) >= 0.0f &&
+                    __fmaf_rn(fsub(1.0f, fadd(u, v)), ad, fadd(r.m, r.m)) >= 0.0f;
     }
     return t >= 0.0f && u >= 0.0f && v >= 0.0f && fadd(u, v) <= 1.0f;
+}
+
+template <bool NEAR = false>
+__device__ __forceinline__ bool tri_test(float ox, float oy, float oz, float dx, float dy, float dz,
+                                         const float4& a, const float4& b, const float4& c,
+                                         float& t, float& u, float& v, bool* nearMiss = nullptr,
+                                         float* slack = nullptr) {
+    const TriTerms r = tri_terms<NEAR>(ox, oy, oz, dx, dy, dz, a, b, c);
+    if (NEAR && slack) { slack[0] = fabsf(r.den); slack[1] = r.m; }
+    return tri_decide<NEAR>(r, t, u, v, nearMiss);
+}
+
+// tri_test for the traversal, which reads t, u, v only of accepted or
+// near-miss triangles: the three divisions (a third of the test) are left out
+// when the numerators show that it is neither.  With x = nu / den exactly
+// and w = x |den|, w < -(2 m + 2^-20 |den|) puts u below -2^-20 (1 - 2^-24) and
+// u |den| + m below 0; the same holds for v.  When neither holds, a negative
+// one of u, v is small, so their sum keeps its relative accuracy, and
+// u + v > 1 + 2^-18 + 4 m / |den| puts the rounded sum above 1 and its slack
+// test below 0.  A comparison with a NaN or an infinite slack is false and
+// leaves the decision to the divisions.  Most of the triangles a ray meets
+// are missed by more than that.
+template <bool NEAR>
+__device__ __forceinline__ bool tri_test_traversal(float ox, float oy, float oz, float dx, float dy, float dz,
+                                                   const float4& a, const float4& b, const float4& c, float& t,
+                                                   float& u, float& v, bool& nearMiss) {
+    const TriTerms r = tri_terms<NEAR>(ox, oy, oz, dx, dy, dz, a, b, c);
+    const float ad = fabsf(r.den);
+    const uint32_t sign = __float_as_uint(r.den) & 0x80000000u;
+    const float wu = __uint_as_float(__float_as_uint(r.nu) ^ sign), wv = __uint_as_float(__float_as_uint(r.nv) ^ sign);
+    const float e = NEAR ? __fmaf_rn(ad, 9.5367431640625e-07f, fadd(r.m, r.m)) : fmul(ad, 9.5367431640625e-07f);
+    nearMiss = false;
+    if (fminf(wu, wv) < -e || fadd(wu, wv) > __fmaf_rn(e, 4.0f, ad)) return false;
+    return tri_decide<NEAR>(r, t, u, v, &nearMiss);
 }
 
 // IntersectTriangle with one reciprocal of the denominator instead of three
@@ -423,10 +469,11 @@ __device__ __forceinline__ bool stage_wait(uint32_t bar, uint32_t parity) {
 
 // Per-lane traversal stack: SMEM entries in shared memory (lane-interleaved),
 // then SPILL entries in local memory.
+// Entry 0 holds kStackEnd, so that a pop needs no test for an empty stack.
 template <int SMEM, int SPILL>
 struct LaneStack {
     int32_t* sh;           // &shared[warp][0][lane]; entry k at sh[k * 32]
-    int32_t spill[SPILL];
+    int32_t spill[SPILL + 1];
     __device__ __forceinline__ void put(uint32_t k, int32_t v) {
         if (k < SMEM) sh[k * 32] = v;
         else spill[k - SMEM] = v;
@@ -434,7 +481,16 @@ struct LaneStack {
     __device__ __forceinline__ int32_t get(uint32_t k) const {
         return k < SMEM ? sh[k * 32] : spill[k - SMEM];
     }
-    static constexpr uint32_t capacity = SMEM + SPILL;
+    static constexpr uint32_t capacity = SMEM + SPILL + 1;
+};
+
+// Trees of fewer than SMEM levels: shared memory alone.
+template <int SMEM>
+struct LaneStack<SMEM, 0> {
+    int32_t* sh;
+    __device__ __forceinline__ void put(uint32_t k, int32_t v) { sh[k * 32] = v; }
+    __device__ __forceinline__ int32_t get(uint32_t k) const { return sh[k * 32]; }
+    static constexpr uint32_t capacity = SMEM;
 };
 
 // One traversal ray in the space of the structure being traversed: its
@@ -645,6 +701,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
 
     LaneStack<SMEM_STACK, SPILL_STACK> st;
     st.sh = &s_stack[warp][0][lane];
+    st.put(0, kStackEnd);
 
     bool live = false;
     bool queueDry = false;          // warp-uniform
@@ -665,9 +722,14 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     unsigned long long nodeCount = 0, triCount = 0;
     const uint32_t nRays = p.n_rays_dev ? min(*p.n_rays_dev, p.n_rays) : p.n_rays;
     const uint32_t nTop = TLAS ? p.n_tlas : p.n_nodes;
-    const int refill = p.refill_steps ? int(p.refill_steps) : 32;
-    const uint32_t refillBelow = p.refill_below;
-    const uint32_t leafWait = ANY ? 0u : p.leaf_wait;
+    // Steps between refills.  Two refinements were measured and left out: a
+    // test of the live lanes at every step, to refill as soon as few are left,
+    // costs more than its earlier refills give back (a million random closest
+    // hits 1,127 against 1,103 us, the camera pass 951 against 940), and
+    // postponing leaf tests until several lanes of the warp are at one holds
+    // back lanes whose loads would overlap (1,168 against 1,112 us at three
+    // lanes, the camera pass 1,025 against 976).
+    const uint32_t burst = p.refill_steps;
 
     // a ray's traversal state from its origin and direction (tmax already set)
     auto beginRay = [&](const float4& o4, const float4& d4, uint32_t nodesHere) {
@@ -683,11 +745,11 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
         }
         hitDist = tmax; second = tmax; hu = 0.0f; hv = 0.0f;
         hitID = -1; hitInst = -1; curInst = -1;
-        node = 0; sp = 0; steps = 0; flags = 0; occl = false; tieSuspect = false;
+        node = 0; sp = 1; steps = 0; flags = 0; occl = false; tieSuspect = false;
         tlasIndex = kTlasInvalid;
         live = true;
         // NaN direction or an empty BVH: miss (bvh.hsh:204, BVH.cpp:107)
-        if (isnan(d4.x) || isnan(d4.y) || isnan(d4.z) || nodesHere == 0) node = INT32_MIN;
+        if (isnan(d4.x) || isnan(d4.y) || isnan(d4.z) || nodesHere == 0) node = kStackEnd;
     };
 
     // scenes: back to the top level, the world-space ray again
@@ -839,29 +901,12 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
         // ---- traverse: a bounded number of steps, then refill again ----
         if (live) {
             const bool anyQ = ANY || (BATCH && laneAny);
-            bool done = node == INT32_MIN;
-            for (int k = 0; k < refill && !done; k++) {
-                // dynamic fetch: leave the burst for a refill once too few lanes
-                // are still traversing (while the queue still has rays)
-                if (refillBelow && !queueDry && uint32_t(__popc(__activemask())) < refillBelow) break;
-                // postponed leaves: a lane at a leaf skips this step while fewer
-                // than leafWait lanes are at leaves and others still descend, so
-                // that the warp's triangle tests run together instead of beside
-                // every node step (the order of each lane's own steps is kept)
-                if (leafWait) {
-                    const bool atLeaf = node < 0 && !(TLAS && sp < tlasIndex);
-                    const uint32_t act = __activemask();
-                    const uint32_t leaves = __ballot_sync(act, atLeaf);
-                    if (atLeaf && uint32_t(__popc(leaves)) < leafWait && leaves != act) continue;
-                }
-                if (++steps > maxSteps) {
-                    flags |= kHitFlagIterCap;
-                    atomicOr(p.error_word, kErrIterationCap);
-                    done = true;
-                    break;
-                }
-                const bool top = TLAS && sp < tlasIndex;
-                if (top) {
+            // the burst ends after `burst` steps or at the ray's step cap
+            const uint32_t lim = min(steps + burst, maxSteps);
+            while (node != kStackEnd) {
+                if (steps >= lim) break;
+                steps++;
+                if (TLAS && sp < tlasIndex) {
                     if (tlasIndex != kTlasInvalid) leaveInstance();
                     if (node < 0) {
                         // CheckInstance: object-space ray, mesh, cull mask
@@ -882,7 +927,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                             node = 0;
                             tlasIndex = sp;
                         } else {
-                            if (sp == 0) { done = true; break; }
                             node = st.get(--sp);
                         }
                         continue;
@@ -891,7 +935,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                 if (BOUNDS && (node < 0 ? uint32_t(~node) >= p.n_tris : uint32_t(node) >= p.n_nodes)) {
                     flags |= kHitFlagOverflow;
                     atomicOr(p.error_word, kErrStackOverflow);
-                    done = true;
+                    node = kStackEnd;
                     break;
                 }
                 if (node < 0) {
@@ -913,8 +957,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         bool nearMiss = false;
                         const bool hit = LOOSE ? tri_test_fast(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(), r.dz(), a, b, c,
                                                                t, u, v)
-                                               : tri_test<TIES && !ANY>(r.ox(), r.oy(), r.oz(), r.dx(), r.dy(),
-                                                                        r.dz(), a, b, c, t, u, v, &nearMiss);
+                                               : tri_test_traversal<TIES && !ANY>(r.ox(), r.oy(), r.oz(), r.dx(),
+                                                                                  r.dy(), r.dz(), a, b, c, t, u, v,
+                                                                                  nearMiss);
                         if (anyQ) {
                             if (hit && t > tmin && t < tmax) { occl = true; end = true; }
                         } else if (hit && t > tmin && t < tmax) {
@@ -929,10 +974,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         }
                         tp++;
                     } while (!end);
-                    if (BOUNDS && (flags & kHitFlagOverflow)) { done = true; break; }
-                    if (anyQ && occl) { done = true; break; }
-                    if (sp == 0) { done = true; break; }
-                    node = st.get(--sp);
+                    if ((BOUNDS && (flags & kHitFlagOverflow)) || (anyQ && occl)) node = kStackEnd;
+                    else node = st.get(--sp);
                 } else {
                     const float4* np = nodes + size_t(node) * 4;
                     const NodeBoxes n = BOUNDS ? load_engine_node(np) : load_node(np);
@@ -965,18 +1008,23 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         if (sp >= st.capacity) {
                             flags |= kHitFlagOverflow;
                             atomicOr(p.error_word, kErrStackOverflow);
-                            done = true;
+                            node = kStackEnd;
                             break;
                         }
                         st.put(sp++, far);
                     } else if (!il && !ir) {
-                        if (sp == 0) { done = true; break; }
                         next = st.get(--sp);
                     }
                     node = next;
                 }
             }
-            if (done) {
+            if (node != kStackEnd && steps >= maxSteps) {
+                // one more visit would exceed the cap
+                flags |= kHitFlagIterCap;
+                atomicOr(p.error_word, kErrIterationCap);
+                node = kStackEnd;
+            }
+            if (node == kStackEnd) {
                 if (anyQ) {
                     uint8_t* occOut = BATCH ? static_cast<uint8_t*>(out) : p.occluded;
                     occOut[rid] = (occl && !(flags & (kHitFlagOverflow | kHitFlagIterCap))) ? 1 : 0;

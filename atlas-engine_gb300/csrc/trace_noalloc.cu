@@ -136,6 +136,7 @@ extern "C" ae_rt_status ae_rt_trace_closest_noalloc(const ae_bvh_node* nodes, ui
     p.error_word = s->scratch + 1;
     p.fetch_counts = nullptr;
     p.max_steps = atlas::rt::dev::default_step_cap(n_nodes);
+    p.refill_steps = atlas::rt::dev::kDefaultRefillSteps;
     uint32_t grid = s->grid;
     const uint32_t needed = (n_rays + kWarps * 32 - 1) / (kWarps * 32);
     if (needed < grid) grid = needed;

@@ -360,14 +360,12 @@ typedef struct ae_rt_config {
     uint32_t threads_per_block;   /* 0 = 128 */
     uint32_t max_steps;           /* traversal step cap per ray (0 = 4 x nodes + 64) */
     uint32_t flags;               /* AE_RT_CFG_COUNT_FETCHES, _NO_NEAR_TIES, _STAGED_RAYS, _APPROXIMATE */
-    uint32_t refill_steps;        /* traversal steps between warp refills (0 = 32) */
+    uint32_t refill_steps;        /* traversal steps between warp refills (0 = 24) */
     uint32_t stack_entries_smem;  /* shared-memory stack entries per lane (0 = 32) */
-    uint32_t refill_below;        /* also refill as soon as fewer than this many lanes of a warp
-                                     are still traversing (1..32; 0 = the default; > 32 = never) */
-    uint32_t leaf_wait;           /* closest-hit traces: a lane that reaches a leaf waits until this
-                                     many lanes of its warp are at leaves (or no lane is at an inner
-                                     node), so that leaf tests run together (0 = never wait;
-                                     scheduling only, results are unchanged) */
+    uint32_t refill_below;        /* 1..32: refill at least every 8 steps (0 or > 32: after
+                                     refill_steps); scheduling only, results are unchanged */
+    uint32_t leaf_wait;           /* accepted and not used: postponing leaf tests slows the
+                                     traversal down in every workload measured */
 } ae_rt_config;
 
 ae_rt_status ae_rt_ctx_create(const ae_rt_config* cfg, ae_rt_ctx** out);
