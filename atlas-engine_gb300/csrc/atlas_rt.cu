@@ -224,6 +224,9 @@ uint32_t MaxSteps(const ae_rt_ctx* ctx, const DeviceMesh& m) {
     return atlas::rt::dev::default_step_cap(m.n_nodes);
 }
 
+// Warps that share the rays of a launch too small to fill the GPU.
+uint32_t SpreadWarps(const ae_rt_ctx* ctx) { return uint32_t(ctx->sm_count) * atlas::rt::dev::kSpreadWarps; }
+
 // Persistent grid for `fn`: SMs x resident CTAs (the configured count, or the
 // kernel's occupancy), never more warps than rays.
 // threads: the block size when it is not the context's (the deep variants,
@@ -240,7 +243,9 @@ uint32_t GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t n_rays, uint32_t
         per_sm = uint32_t(occ > 0 ? occ : 1);
     }
     uint32_t grid = uint32_t(ctx->sm_count) * per_sm;
-    const uint32_t needed = (n_rays + threads - 1) / threads;
+    // warps: one per 32 rays, or enough to spread few rays over the GPU
+    const uint32_t warps = std::max((n_rays + 31) / 32, std::min(n_rays, SpreadWarps(ctx)));
+    const uint32_t needed = (warps + threads / 32 - 1) / (threads / 32);
     if (needed < grid) grid = needed;
     return grid == 0 ? 1 : grid;
 }
@@ -263,6 +268,7 @@ ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStre
     AE_CUDA(ctx, cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
+    p.spread_warps = SpreadWarps(ctx);
     const bool deep = depth > uint32_t(kStackEntries) && mode != MODE_BATCH;
     void* fn = deep ? PickDeep(any, mode, ties && ctx->near_ties)
                     : PickKernelShape(ctx->shape, depth, any, ctx->count_fetches, mode, ties && ctx->near_ties,
@@ -796,6 +802,7 @@ TraceParams BatchParams(ae_rt_ctx* ctx, const atlas::rt::dev::BatchDesc* d_batch
     p.batches = d_batches;
     p.n_batches = n;
     p.refill_steps = ctx->refill_steps;
+    p.spread_warps = SpreadWarps(ctx);
     p.max_steps = 0xffffffffu;
     return p;
 }

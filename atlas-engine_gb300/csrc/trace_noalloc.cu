@@ -18,6 +18,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 namespace {
@@ -42,6 +43,7 @@ struct DeviceSetup {
     bool ready = false;
     uint32_t* scratch = nullptr;   // device address of g_trace_scratch on this device
     uint32_t grid = 0;             // persistent grid: SMs x resident CTAs
+    uint32_t spread = 0;           // warps that share the rays of a small launch
 };
 
 std::mutex g_setup_mutex;
@@ -85,6 +87,7 @@ ae_rt_status SetupDevice(int dev, DeviceSetup** out) {
         }
         s.scratch = static_cast<uint32_t*>(ptr);
         s.grid = uint32_t(sms) * uint32_t(blocks > 0 ? blocks : 1);
+        s.spread = uint32_t(sms) * atlas::rt::dev::kSpreadWarps;
         s.ready = true;
     }
     *out = &s;
@@ -137,8 +140,10 @@ extern "C" ae_rt_status ae_rt_trace_closest_noalloc(const ae_bvh_node* nodes, ui
     p.fetch_counts = nullptr;
     p.max_steps = atlas::rt::dev::default_step_cap(n_nodes);
     p.refill_steps = atlas::rt::dev::kDefaultRefillSteps;
+    p.spread_warps = s->spread;
     uint32_t grid = s->grid;
-    const uint32_t needed = (n_rays + kWarps * 32 - 1) / (kWarps * 32);
+    const uint32_t warps = std::max((n_rays + 31) / 32, std::min(n_rays, s->spread));
+    const uint32_t needed = (warps + kWarps - 1) / kWarps;
     if (needed < grid) grid = needed;
     void* args[] = { &p };
     if (cudaLaunchKernel(NoAllocKernel(), dim3(grid), dim3(kWarps * 32), args, 0, cs) != cudaSuccess) {

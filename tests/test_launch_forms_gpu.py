@@ -1,0 +1,84 @@
+"""The traversal's launch forms: stack variants chosen by tree depth, and
+launches of few rays, which fill only some lanes of each warp.  Every form
+returns the same bits: the oracle's nearest triangle for the stacks, the
+records of a full launch for the first rays of a small one."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import atlas_rt
+import pyoracle
+from atlas_rt import BVH, _native, scenes
+from test_trace_gpu import chain_bvh, packed
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("entries", [30, 31, 32, 33, 126, 127, 128, 129])
+def test_stack_variants_at_their_edges(ctx, entries):
+    """A chain that needs exactly this many stack entries, around the shared
+    memory alone (31 and the end marker), the usual 128 and the deep stack."""
+    nodes, tris = chain_bvh(entries + 1)
+    mid = ctx.upload_mesh(nodes, tris)
+    rays8 = scenes.rays8(np.tile(np.array([[0.5, 0.5, -1.0]], np.float32), (70, 1)),
+                         np.tile(np.array([[0.01, -0.02, 1.0]], np.float32), (70, 1)), 0.0, 1e4)
+    hits = ctx.trace_closest(mid, packed(rays8), 0.0, 1e4)
+    ptr, tuv = pyoracle.closest_glsl(nodes.view(np.float32).reshape(-1, 16), tris, rays8)
+    assert np.array_equal(hits["triPtr"], ptr) and (ptr == entries).all()
+    assert np.array_equal(hits["t"].view(np.uint32), tuv[:, 0].view(np.uint32))
+    assert (hits["flags"] & 0xC == 0).all()
+    assert ctx.trace_any(mid, packed(rays8), 0.0, 1e4).all()
+
+
+@pytest.fixture(scope="module")
+def few():
+    """A mesh, a two-instance scene of it, 60,000 rays and their full-launch results."""
+    import torch
+    c = atlas_rt.Context(device=0)
+    b = BVH(scenes.random_triangles(9000, seed=11))
+    gt = b.pack_triangles()
+    mid = c.upload_mesh(b.nodes, gt)
+    lo, hi = atlas_rt.mesh_bounds(b)
+    models = [np.eye(4), np.diag([1.5, 0.7, 1.1, 1.0])]
+    c.scene_build(np.array([atlas_rt.make_instance(m, mid, atlas_rt.MASK_ALL) for m in models]),
+                  np.array([atlas_rt.transform_aabb(lo, hi, m) for m in models]))
+    rays = torch.from_numpy(scenes.pack_rays(*scenes.sphere_rays(60000, seed=12))).cuda()
+    d = {"ctx": c, "mid": mid, "rays": rays, "torch": torch, "bvh": b, "gt": gt}
+    d["full"] = {k: run(d, k, len(rays)) for k in ("closest", "any", "scene", "queue", "noalloc")}
+    yield d
+    c.close()
+
+
+def run(d, kind, n):
+    c, rays, torch = d["ctx"], d["rays"], d["torch"]
+    hits = torch.full((len(rays), 8), float("nan"), device="cuda")
+    occ = torch.full((len(rays),), 7, dtype=torch.uint8, device="cuda")
+    if kind == "closest":
+        c.trace_closest(d["mid"], rays, 1e-4, 10.0, out=hits, n_rays=n)
+    elif kind == "any":
+        c.trace_any(d["mid"], rays, 1e-4, 10.0, out=occ, n_rays=n)
+    elif kind == "scene":
+        c.trace_scene_closest(rays, 1e-4, 10.0, out=hits, n_rays=n)
+    elif kind == "queue":       # the count is read on the device
+        c.trace_closest_queue(d["mid"], rays, torch.tensor([n], dtype=torch.int32, device="cuda"), len(rays), 1e-4,
+                              10.0, hits)
+    else:
+        nodes, tris = torch.from_numpy(d["bvh"].nodes_f32.copy()).cuda(), torch.from_numpy(d["gt"]).cuda()
+        assert _native.lib().ae_rt_trace_closest_noalloc(
+            nodes.data_ptr(), len(d["bvh"].nodes), tris.data_ptr(), len(d["gt"]), rays.data_ptr(), n, C.c_float(1e-4),
+            C.c_float(10.0), hits.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+    c.synchronize()
+    out = occ if kind == "any" else hits.view(torch.int32)
+    return out.cpu().numpy()
+
+
+# around one ray, one warp, one warp's share on every SM (8 warps of 152 SMs) and 32 lanes there
+@pytest.mark.parametrize("kind", ["closest", "any", "scene", "queue", "noalloc"])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1215, 1216, 1217, 2433, 38911, 38912, 38913])
+def test_few_rays_give_the_full_launch_records(few, kind, n):
+    got, full = run(few, kind, n), few["full"][kind]
+    untouched = np.float32("nan").view(np.int32) if kind != "any" else 7
+    assert np.array_equal(got[:n], full[:n])
+    assert (got[n:] == untouched).all()
