@@ -224,14 +224,13 @@ uint32_t MaxSteps(const ae_rt_ctx* ctx, const DeviceMesh& m) {
     return atlas::rt::dev::default_step_cap(m.n_nodes);
 }
 
-// Warps that share the rays of a launch too small to fill the GPU.
-uint32_t SpreadWarps(const ae_rt_ctx* ctx) { return uint32_t(ctx->sm_count) * atlas::rt::dev::kSpreadWarps; }
+}  // namespace
 
-// Persistent grid for `fn`: SMs x resident CTAs (the configured count, or the
-// kernel's occupancy), never more warps than rays.
-// threads: the block size when it is not the context's (the deep variants,
-// sized by their occupancy alone).
-uint32_t GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t n_rays, uint32_t threads = 0) {
+uint32_t atlas::rt::host::SpreadWarps(const ae_rt_ctx* ctx) {
+    return uint32_t(ctx->sm_count) * atlas::rt::dev::kSpreadWarps;
+}
+
+uint32_t atlas::rt::host::GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t n_rays, uint32_t threads) {
     uint32_t per_sm = threads ? 0u : ctx->blocks_per_sm;
     if (threads == 0) threads = ctx->threads;
     if (per_sm == 0) {
@@ -250,13 +249,14 @@ uint32_t GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t n_rays, uint32_t
     return grid == 0 ? 1 : grid;
 }
 
-// Work-counter words of the context's launches, used in rotation so that
-// launches on different streams (up to kWorkSlots at a time) can overlap.
-constexpr uint32_t kWorkSlots = 6;
-uint32_t* WorkCounter(ae_rt_ctx* ctx) {
+cudaError_t atlas::rt::host::NextWorkCounter(ae_rt_ctx* ctx, cudaStream_t s, uint32_t** counter) {
+    constexpr uint32_t kWorkSlots = 6;
     const uint32_t k = ctx->next_work_slot++ % kWorkSlots;
-    return ctx->d_counter + (k == 0 ? 0u : k + 1u);          // word 1 is the error word
+    *counter = ctx->d_counter + (k == 0 ? 0u : k + 1u);      // word 1 is the error word
+    return cudaMemsetAsync(*counter, 0, sizeof(uint32_t), s);
 }
+
+namespace {
 
 // depth: stack entries the launch's trees can need (batched launches hold
 // kStackEntries at most and report overflow beyond).
@@ -264,8 +264,7 @@ uint32_t* WorkCounter(ae_rt_ctx* ctx) {
 // within kStackEntries, exact, no counters: Trace checks this).
 ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStream_t s, bool ties, uint32_t depth,
                     bool camera = false) {
-    if (p.work_counter == ctx->d_counter) p.work_counter = WorkCounter(ctx);
-    AE_CUDA(ctx, cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s));
+    AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
@@ -354,7 +353,6 @@ ae_rt_status Trace(ae_rt_ctx* ctx, bool any, int32_t mesh_id, const ae_packed_ra
     p.tmax = tmax;
     p.hits = any ? nullptr : static_cast<float4*>(d_out);
     p.occluded = any ? static_cast<uint8_t*>(d_out) : nullptr;
-    p.work_counter = ctx->d_counter;
     p.error_word = ctx->d_counter + 1;
     p.fetch_counts = ctx->d_fetch;
     p.max_steps = scene ? (ctx->max_steps_cfg ? ctx->max_steps_cfg : ctx->scene_steps) : MaxSteps(ctx, m);
@@ -792,11 +790,9 @@ ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32
     return AE_RT_OK;
 }
 
-TraceParams BatchParams(ae_rt_ctx* ctx, const atlas::rt::dev::BatchDesc* d_batches, uint32_t n, uint32_t total,
-                        uint32_t* counter) {
+TraceParams BatchParams(ae_rt_ctx* ctx, const atlas::rt::dev::BatchDesc* d_batches, uint32_t n, uint32_t total) {
     TraceParams p{};
     p.n_rays = total;
-    p.work_counter = counter;
     p.error_word = ctx->d_counter + 1;
     p.fetch_counts = ctx->d_fetch;
     p.batches = d_batches;
@@ -824,7 +820,7 @@ ae_rt_status ae_rt_trace_batched(ae_rt_ctx* ctx, const ae_batch_desc* batches, u
     AE_CUDA(ctx, cudaMemcpyAsync(ctx->batch_table.ptr, table.data(), table.size() * sizeof(table[0]),
                                  cudaMemcpyHostToDevice, s));
     TraceParams p = BatchParams(ctx, static_cast<atlas::rt::dev::BatchDesc*>(ctx->batch_table.ptr), n_batches,
-                                total, ctx->d_counter);
+                                total);
     return Launch(ctx, false, MODE_BATCH, p, s, true, depth);
 }
 
@@ -851,10 +847,11 @@ ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batche
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        TraceParams p = BatchParams(ctx, plan->d_batches, n_batches, total, plan->d_counter);
-        cudaError_t le = cudaMemsetAsync(plan->d_counter, 0, sizeof(uint32_t), cap);
+        TraceParams p = BatchParams(ctx, plan->d_batches, n_batches, total);
+        p.work_counter = plan->d_counter;
         void* args[] = { &p };
         void* fn = PickKernelShape(ctx->shape, depth, false, false, MODE_BATCH, ctx->near_ties);
+        cudaError_t le = cudaMemsetAsync(plan->d_counter, 0, sizeof(uint32_t), cap);
         if (le == cudaSuccess)
             le = cudaLaunchKernel(fn, dim3(GridFor(ctx, fn, total)), dim3(ctx->threads), args, 0, cap);
         e = cudaStreamEndCapture(cap, &plan->graph);

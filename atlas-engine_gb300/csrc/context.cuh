@@ -160,6 +160,18 @@ inline bool IsDevicePointer(const void* p) {
 }
 
 
+// The work counter of the context's next persistent launch, zeroed on its
+// stream: six in rotation, so that launches on different streams can overlap.
+cudaError_t NextWorkCounter(ae_rt_ctx* ctx, cudaStream_t s, uint32_t** counter);
+
+// Persistent grid for kernel `fn`: SMs x resident CTAs (the configured count,
+// or the kernel's occupancy), never more warps than rays.  threads: the block
+// size when it is not the context's (then the occupancy alone counts).
+uint32_t GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t n_rays, uint32_t threads = 0);
+
+// Warps that share the rays of a launch too small to fill the GPU.
+uint32_t SpreadWarps(const ae_rt_ctx* ctx);
+
 // Queue-driven trace over the context's two-level scene (rays, out and count
 // in device memory), for the other translation units.
 // Closest / any-hit trace of a scene queue for the library's own consumers

@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "camera.cuh"
+#include "texture.cuh"
 
 namespace atlas::rt::dev {
 
@@ -79,6 +80,11 @@ struct TraceParams {
     uint32_t refill_steps;       // traversal steps between warp refills
     uint32_t spread_warps;       // warps that share the rays of a small launch (kSpreadWarps an SM)
     uint32_t per_ray_tmax;       // nonzero: a ray's tmax is its PackedRay hit.x (shadow queues)
+    // transparency launches (OPACITY)
+    const float* materials;      // GPUMaterial (23 words), may be null (opacity 1)
+    uint32_t n_materials;
+    TexTable textures;
+    float* transparency;         // one float per ray (any hit)
     CameraParams cam;            // the camera variant: ray i is camera_ray(cam, i), `rays` unused
 };
 
@@ -662,6 +668,15 @@ __device__ __forceinline__ uint32_t find_batch(const BatchDesc* b, uint32_t n, u
     return lo;
 }
 
+// `tri.opacity < 0.0 ? GetOpacity(tri, sol.yz, materialOffset, 0) : tri.opacity`
+// (out of line: the texture path is rare and would take the registers of the
+// whole traversal).
+static __device__ __noinline__ float texture_opacity(const float* materials, uint32_t n_materials, const uint8_t* pool,
+                                              const TexDesc* desc, uint32_t n_tex, const float4* d0, int32_t matOffset,
+                                              float u, float v) {
+    return get_opacity(materials, n_materials, TexTable{ pool, desc, n_tex }, __ldg(d0), matOffset, u, v);
+}
+
 // ANY: HitAny instead of HitClosest.  COUNT: per-launch node / triangle fetch
 // totals.  MODE_SCENE: two-level traversal over instances (CheckInstance,
 // bvh.hsh:172-189, with the TLAS/BLAS switch keyed on the stack depth at which
@@ -686,16 +701,28 @@ __device__ __forceinline__ uint32_t find_batch(const BatchDesc* b, uint32_t n, u
 // tri_test_fast, for consumers whose results are Monte Carlo estimates
 // (AE_RT_CFG_APPROXIMATE), not the shader's bit for bit.
 //
+// OPACITY: the transparency variants HitClosestTransparency (bvh.hsh:275-357,
+// + CheckLeafClosestTransparency :106-138) and HitAnyTransparency
+// (bvh.hsh:443-524, + CheckLeafTransparency :140-170).  Leaves read the
+// 96-byte shading triangle (UnpackTriangle, common.hsh:17-44): its vertices,
+// endOfNode = d1.z > 0 and opacity = d2.w or GetOpacity.  Closest: a hit counts
+// only where its opacity is > 0.  Any: every accepted triangle multiplies the
+// leaf's running transparency, which starts from the current value; the
+// leaf's result multiplies the current value again (bvh.hsh:500), values
+// below 1e-6 become 0, and the traversal ends at 0.
+//
 // CAMERA: ray i is the camera ray of queue slot i (camera_ray), made by the
 // lane that takes it, instead of a load from a ray buffer written by a
 // separate ray-generation launch.
 template <bool ANY, bool COUNT, int MODE, int WARPS, int SMEM_STACK, int SPILL_STACK, int MIN_BLOCKS,
-          bool BOUNDS = false, bool TIES = true, int STAGE = 0, bool LOOSE = false, bool CAMERA = false>
+          bool BOUNDS = false, bool TIES = true, int STAGE = 0, bool LOOSE = false, bool CAMERA = false,
+          bool OPACITY = false>
 __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TraceParams p) {
     constexpr bool TLAS = MODE == MODE_SCENE;
     constexpr bool BATCH = MODE == MODE_BATCH;
     static_assert(STAGE == 0 || (!BATCH && !BOUNDS), "staged rays: single-mesh and scene launches only");
     static_assert(!LOOSE || (!TIES && !BOUNDS), "loose traversal: no near-tie flag, uploaded nodes");
+    static_assert(!OPACITY || (TLAS && !TIES && !LOOSE && !COUNT && !BOUNDS && STAGE == 0), "transparency: exact scenes");
     static_assert(!CAMERA || (MODE == MODE_MESH && STAGE == 0 && !ANY), "camera rays: single-mesh closest hits");
     __shared__ int32_t s_stack[WARPS][SMEM_STACK][32];
     // scenes: the world-space ray of each lane while it is inside an instance
@@ -729,6 +756,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     uint32_t maxSteps = p.max_steps;
     void* out = nullptr;            // batched: the lane's result array
     unsigned long long nodeCount = 0, triCount = 0;
+    float transparency = 1.0f;      // OPACITY, any hit
+    int32_t matOffset = 0;          // OPACITY: of the current instance
     const uint32_t nRays = p.n_rays_dev ? min(*p.n_rays_dev, p.n_rays) : p.n_rays;
     const uint32_t nTop = TLAS ? p.n_tlas : p.n_nodes;
     // Steps between refills.  Two refinements were measured and left out: a
@@ -759,6 +788,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
         hitID = -1; hitInst = -1; curInst = -1;
         node = 0; sp = 1; steps = 0; flags = 0; occl = false; tieSuspect = false;
         tlasIndex = kTlasInvalid;
+        transparency = 1.0f;
         live = true;
         // NaN direction or an empty BVH: miss (bvh.hsh:204, BVH.cpp:107)
         if (isnan(d4.x) || isnan(d4.y) || isnan(d4.z) || nodesHere == 0) node = kStackEnd;
@@ -930,12 +960,14 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         MeshDesc m{};
                         if (enter) {
                             m = p.meshes[__float_as_int(c3.x)];
-                            enter = m.n_nodes > 0;     // an empty BLAS has no root to visit
+                            // an empty BLAS has no root to visit
+                            enter = m.n_nodes > 0 && (!OPACITY || m.shading);
                         }
                         if (enter) {
                             r = transform_ray(r, c0, c1, c2);
                             nodes = m.nodes;
-                            blasTris = m.tris;
+                            blasTris = OPACITY ? m.shading : m.tris;
+                            if (OPACITY) matOffset = __float_as_int(c3.y);
                             node = 0;
                             tlasIndex = sp;
                         } else {
@@ -954,16 +986,22 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                     // Leaf: contiguous triangles up to the end-of-node flag.
                     int32_t tp = ~node;
                     bool end = false;
+                    float leafTransparency = transparency;
                     do {
                         if (BOUNDS && uint32_t(tp) >= p.n_tris) {
                             flags |= kHitFlagOverflow;
                             atomicOr(p.error_word, kErrStackOverflow);
                             break;
                         }
-                        const float4 a = ldg4(blasTris + size_t(tp) * 3);
-                        const float4 b = ldg4(blasTris + size_t(tp) * 3 + 1);
-                        const float4 c = ldg4(blasTris + size_t(tp) * 3 + 2);
-                        end = a.w > 0.0f;
+                        const float4* tri = blasTris + size_t(tp) * (OPACITY ? 6 : 3);
+                        const float4 a = ldg4(tri), b = ldg4(tri + 1), c = ldg4(tri + 2);
+                        float opacity = 1.0f;
+                        if (OPACITY) {
+                            end = ldg4(tri + 4).z > 0.0f;
+                            opacity = ldg4(tri + 5).w;
+                        } else {
+                            end = a.w > 0.0f;
+                        }
                         if (COUNT) triCount++;
                         float t, u, v;
                         bool nearMiss = false;
@@ -972,7 +1010,18 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                                                : tri_test_traversal<TIES && !ANY>(r.ox(), r.oy(), r.oz(), r.dx(),
                                                                                   r.dy(), r.dz(), a, b, c, t, u, v,
                                                                                   nearMiss);
-                        if (anyQ) {
+                        if (OPACITY) {
+                            if (hit && t > tmin && t < (ANY ? tmax : hitDist)) {
+                                if (opacity < 0.0f)
+                                    opacity = texture_opacity(p.materials, p.n_materials, p.textures.pool,
+                                                              p.textures.desc, p.textures.n, tri + 3, matOffset, u, v);
+                                if (ANY) {
+                                    leafTransparency = fmul(leafTransparency, fsub(1.0f, opacity));
+                                } else if (opacity > 0.0f) {
+                                    hitDist = t; hitID = tp; hu = u; hv = v; hitInst = curInst;
+                                }
+                            }
+                        } else if (anyQ) {
                             if (hit && t > tmin && t < tmax) { occl = true; end = true; }
                         } else if (hit && t > tmin && t < tmax) {
                             if (t < hitDist) {
@@ -986,6 +1035,11 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         }
                         tp++;
                     } while (!end);
+                    if (OPACITY && ANY) {
+                        transparency = fmul(transparency, leafTransparency);
+                        if (transparency < 0.000001f) transparency = 0.0f;
+                        occl = !(transparency > 0.0f);
+                    }
                     if ((BOUNDS && (flags & kHitFlagOverflow)) || (anyQ && occl)) node = kStackEnd;
                     else node = st.get(--sp);
                 } else {
@@ -1037,13 +1091,16 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                 node = kStackEnd;
             }
             if (node == kStackEnd) {
-                if (anyQ) {
+                if (OPACITY && ANY) {
+                    p.transparency[rid] = transparency;
+                } else if (anyQ) {
                     uint8_t* occOut = BATCH ? static_cast<uint8_t*>(out) : p.occluded;
                     occOut[rid] = (occl && !(flags & (kHitFlagOverflow | kHitFlagIterCap))) ? 1 : 0;
                 } else {
                     const bool hit = hitID >= 0;
                     uint32_t f = flags | (hit ? kHitFlagHit : 0u);
-                    if (TIES ? (hit && fsub(second, hitDist) <= fmul(kTieWindow, hitDist)) || tieSuspect
+                    if (OPACITY) second = tmax;
+                    else if (TIES ? (hit && fsub(second, hitDist) <= fmul(kTieWindow, hitDist)) || tieSuspect
                              : hit && fsub(second, hitDist) <= fmul(1e-6f, hitDist))
                         f |= kHitFlagNearTie;
                     float4* hp = (BATCH ? static_cast<float4*>(out) : p.hits) + size_t(rid) * 2;

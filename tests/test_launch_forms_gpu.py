@@ -82,3 +82,34 @@ def test_few_rays_give_the_full_launch_records(few, kind, n):
     untouched = np.float32("nan").view(np.int32) if kind != "any" else 7
     assert np.array_equal(got[:n], full[:n])
     assert (got[n:] == untouched).all()
+
+
+@pytest.mark.parametrize("entries", [29, 30, 31, 126])
+def test_transparency_stacks_on_an_opaque_chain(entries):
+    """The transparency traversal of an opaque scene is the opaque one, around
+    the depth where its stack leaves shared memory (one top-level entry more
+    than the chain's), and for launches of one ray to several hundred."""
+    nodes, tris = chain_bvh(entries + 1)
+    shading = np.zeros((len(tris), 24), np.float32)
+    shading[:, 0:12] = tris
+    shading[:, [3, 7, 11]] = 0.0
+    shading[:, 18], shading[:, 23] = 1.0, 1.0
+    c = atlas_rt.Context(device=0)
+    try:
+        mid = c.upload_mesh(nodes, tris, shading)
+        c.scene_build(np.array([atlas_rt.make_instance(np.eye(4), mid, atlas_rt.MASK_ALL)]),
+                      np.array([[-1.0, -1.0, 1.0, 3.0, 3.0, entries + 1.0]], np.float32))
+        rng = np.random.default_rng(entries)
+        o = np.concatenate([rng.uniform(-1.5, 3.5, (700, 2)), np.full((700, 1), -1.0)], 1).astype(np.float32)
+        rays = scenes.pack_rays(o, np.tile(np.array([[0.01, -0.02, 1.0]], np.float32), (700, 1)))
+        want, occ = c.trace_scene_closest(rays, 0.0, 1e4), c.trace_scene_any(rays, 0.0, 1e4)
+        assert 50 < (want["triPtr"] >= 0).sum() < 650
+        for n in (1, 33, 700):
+            got = c.trace_scene_closest_transparency(rays[:n].copy(), 0.0, 1e4)
+            for k in ("t", "triPtr", "instance", "u", "v"):
+                assert np.array_equal(got[k].view(np.uint32), want[k][:n].view(np.uint32)), (n, k)
+            assert (got["tSecond"] == 1e4).all()
+            vis = c.trace_scene_any_transparency(rays[:n].copy(), 0.0, 1e4)
+            assert np.array_equal(vis, 1.0 - occ[:n].astype(np.float32))
+    finally:
+        c.close()
