@@ -23,6 +23,7 @@
 #include "context.cuh"
 #include "trace_kernels.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 using namespace atlas::rt::host;
@@ -30,6 +31,10 @@ using namespace atlas::rt::host;
 namespace {
 
 constexpr uint32_t kRetestStack = 128;
+constexpr int kRetestSmem = 32;            // of them in shared memory
+constexpr int kRetestThreads = 128;
+constexpr int kRetestBlocks = 4;           // CTAs an SM
+constexpr int kRetestBatch = 4;            // lanes that test their triangles together
 constexpr double kSecondWindow = 1e-5;     // ten times the 1e-6 of a near tie
 
 // The farthest distance that can still matter: best + |best| kSecondWindow
@@ -113,14 +118,18 @@ __device__ __forceinline__ bool tri64(const double o[3], const double d[3], cons
     const double den = dot3(q, e0);
     const double nt = dot3(p, e1), nu = dot3(q, s), nv = dot3(p, d);
     const double ad = fabs(den);
+    bool inside = false;
     if (ad > 1e-200 && ad < 1e200) {
         const double sg = den < 0.0 ? -1.0 : 1.0;
         const double wt = nt * sg, wu = nu * sg, wv = nv * sg;      // exact: sign flips
         const double m = 1e-12 * ad;
         if (wu < -m || wv < -m || wt < -m || (wu >= 0.0 && wv >= 0.0 && wu + wv > ad + m) || wt > bound * (ad + m))
             return false;
+        // clearly inside by the same margins: the quotients u and v would pass
+        inside = wu > m && wv > m && wu + wv < ad - m;
     }
     t = __ddiv_rn(nt, den);
+    if (inside) return t >= 0.0;
     const double u = __ddiv_rn(nu, den);
     const double v = __ddiv_rn(nv, den);
     return t >= 0.0 && u >= 0.0 && v >= 0.0 && da(u, v) <= 1.0;
@@ -168,33 +177,75 @@ __global__ void retest_compact_kernel(RetestParams p) {
 }
 
 // Pass 2: the double-precision search for every listed ray.
-__global__ void retest_kernel(RetestParams p) {
+//
+// Double-precision instructions issue at a small fraction of the FP32 rate
+// whatever the number of lanes that take part, and a search makes about two
+// triangle tests among forty node visits.  So a lane whose triangle passes
+// the single-precision screen waits with it until kRetestBatch lanes of its
+// warp hold one (or no lane can go on without), and they test together; the
+// pruning bound is kept rounded up in single precision, so that a node visit
+// takes no double-precision operation.
+__global__ void __launch_bounds__(kRetestThreads, kRetestBlocks) retest_kernel(RetestParams p) {
+    using namespace atlas::rt::dev;
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ int32_t s_stack[kRetestThreads / 32][kRetestSmem][32];
     const uint32_t count = *p.n_retested;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += stride) {
-        const uint32_t i = p.list[j];
-        ae_hit_f64 r;
-        r.reserved[0] = r.reserved[1] = 0;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t warps = gridDim.x * (kRetestThreads / 32);
+    LaneStack<kRetestSmem, int(kRetestStack) - kRetestSmem> st;
+    st.sh = &s_stack[warp][0][lane];
+    st.put(0, kStackEnd);
+    const float tminf = __double2float_rd(p.tmin);
+
+    // consecutive listed rays go to different warps: neighbours on the list are
+    // neighbours on screen, and the few long searches should not share a warp
+    uint32_t j = lane * warps + blockIdx.x * (kRetestThreads / 32) + warp;
+    uint32_t i = 0, sp = 1, steps = 0;
+    float of[3] = { 0, 0, 0 }, df[3] = { 0, 0, 0 }, yf[3] = { 0, 0, 0 };
+    double best = INFINITY, second = INFINITY, bound = INFINITY;
+    float boundf = INFINITY;
+    int32_t bi = -1, node = kStackEnd, tp = -1;      // tp: the current triangle while inside a leaf
+    bool have = false, waits = false, end = false, bad = false;
+    auto take = [&]() {
+        have = j < count;
+        if (!have) return;
+        i = p.list[j];
+        j += warps * 32u;
         const float4 o4 = p.rays[size_t(i) * 3], d4 = p.rays[size_t(i) * 3 + 1];
-        const double o[3] = { o4.x, o4.y, o4.z }, d[3] = { d4.x, d4.y, d4.z };
-        const float of[3] = { o4.x, o4.y, o4.z }, df[3] = { d4.x, d4.y, d4.z };
-        const float yf[3] = { __frcp_rn(d4.x), __frcp_rn(d4.y), __frcp_rn(d4.z) };
-        const float tminf = __double2float_rd(p.tmin);
-        double best = INFINITY, second = INFINITY;
-        int32_t bi = -1;
-        int32_t stack[kRetestStack];
-        uint32_t sp = 0, steps = 0;
-        int32_t node = 0;
-        bool bad = false;
-        while (true) {
-            if (++steps > p.max_steps) { bad = true; atomicOr(p.error_word, atlas::rt::dev::kErrIterationCap); break; }
-            if (node < 0) {
-                int32_t tp = ~node;
-                bool end = false;
+        of[0] = o4.x; of[1] = o4.y; of[2] = o4.z;
+        df[0] = d4.x; df[1] = d4.y; df[2] = d4.z;
+        for (int k = 0; k < 3; k++) yf[k] = __frcp_rn(df[k]);
+        best = INFINITY;
+        second = INFINITY;
+        bound = p.tmax;
+        boundf = __double2float_ru(bound);
+        bi = -1;
+        node = 0;
+        tp = -1;
+        sp = 1;
+        steps = 0;
+        waits = false;
+        bad = false;
+    };
+    auto give_up = [&]() {
+        bad = true;
+        node = kStackEnd;
+        waits = false;
+    };
+    take();
+    for (;;) {
+        const uint32_t active = __ballot_sync(kFull, have);
+        if (!active) break;
+        if (have && !waits) {
+            if (tp < 0 && ++steps > p.max_steps) {
+                atomicOr(p.error_word, kErrIterationCap);
+                give_up();
+            } else if (node < 0) {
+                if (tp < 0) tp = ~node;
                 do {
-                    if (uint32_t(tp) >= p.n_tris) { bad = true; break; }
-                    const float4 A = __ldg(p.tris + size_t(tp) * 3), B = __ldg(p.tris + size_t(tp) * 3 + 1),
-                                 C = __ldg(p.tris + size_t(tp) * 3 + 2);
+                    if (uint32_t(tp) >= p.n_tris) { give_up(); break; }
+                    const float4* tq = p.tris + size_t(tp) * 3;
+                    const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
                     end = A.w > 0.0f;
                     // single-precision screen: the FP32 barycentrics are within m / |den|
                     // of the exact ones (the near-tie slack), so a triangle outside its
@@ -202,62 +253,77 @@ __global__ void retest_kernel(RetestParams p) {
                     // by more than m / |den| -- far more than the double test's rounding
                     float t32, u32, v32, sl[2];
                     bool near32 = true;
-                    (void)atlas::rt::dev::tri_test<true>(of[0], of[1], of[2], df[0], df[1], df[2], A, B, C, t32, u32,
-                                                         v32, &near32, sl);
+                    (void)tri_test<true>(of[0], of[1], of[2], df[0], df[1], df[2], A, B, C, t32, u32, v32, &near32, sl);
                     const float ad = sl[0], m2 = 2.0f * sl[1];
                     const bool outside = ad > 2.0f * m2 && isfinite(u32) && isfinite(v32) &&
                                          !(__fmaf_rn(u32, ad, m2) >= 0.0f && __fmaf_rn(v32, ad, m2) >= 0.0f &&
                                            __fmaf_rn(1.0f - (u32 + v32), ad, 2.0f * m2) >= 0.0f);
-                    double t;
-                    if (!outside && tri64(o, d, A, B, C, fmin(fmin(p.tmax, second), second_limit(best)), t) && t > p.tmin &&
-                        t < p.tmax &&
-                        !(bi >= 0 && t == best && same_triangle(p.tris + size_t(bi) * 3, A, B, C))) {
-                        if (t < best || (t == best && tp < bi)) {
-                            if (tp != bi) second = best;
-                            best = t;
-                            bi = tp;
-                        } else if (t < second && tp != bi) {
-                            second = t;
-                        }
-                    }
-                    tp++;
-                } while (!end);
-                if (bad || sp == 0) break;
-                node = stack[--sp];
-                continue;
-            }
-            if (uint32_t(node) >= p.n_nodes) { bad = true; break; }
-            const float4* np = p.nodes + size_t(node) * 4;
-            using atlas::rt::dev::lo2;
-            using atlas::rt::dev::hi2;
-            const atlas::rt::dev::NodeBoxes n = atlas::rt::dev::load_node(np);
-            // prune by the second distance, and by the window past the nearest
-            // beyond which a second distance is not reported
-            const double bound = fmin(fmin(p.tmax, second), second_limit(best));
-            const float boundf = __double2float_ru(bound);
-            const bool il = box32(of, df, yf, lo2(n.l_lo_xy), hi2(n.l_lo_xy), lo2(n.l_z), lo2(n.l_hi_xy),
-                                  hi2(n.l_hi_xy), hi2(n.l_z), tminf, boundf);
-            const bool ir = box32(of, df, yf, lo2(n.r_lo_xy), hi2(n.r_lo_xy), lo2(n.r_z), lo2(n.r_hi_xy),
-                                  hi2(n.r_hi_xy), hi2(n.r_z), tminf, boundf);
-            const int32_t l = n.lptr, rr = n.rptr;
-            if (il && ir) {
-                if (sp >= kRetestStack) { bad = true; atomicOr(p.error_word, atlas::rt::dev::kErrStackOverflow); break; }
-                stack[sp++] = rr;
-                node = l;
-            } else if (il) {
-                node = l;
-            } else if (ir) {
-                node = rr;
+                    waits = !outside;
+                    if (!waits) tp++;
+                } while (!waits && !end);
+                if (!waits && !bad) {
+                    tp = -1;
+                    node = st.get(--sp);
+                }
+            } else if (uint32_t(node) >= p.n_nodes) {
+                give_up();
             } else {
-                if (sp == 0) break;
-                node = stack[--sp];
+                const NodeBoxes n = load_node(p.nodes + size_t(node) * 4);
+                const bool il = box32(of, df, yf, lo2(n.l_lo_xy), hi2(n.l_lo_xy), lo2(n.l_z), lo2(n.l_hi_xy),
+                                      hi2(n.l_hi_xy), hi2(n.l_z), tminf, boundf);
+                const bool ir = box32(of, df, yf, lo2(n.r_lo_xy), hi2(n.r_lo_xy), lo2(n.r_z), lo2(n.r_hi_xy),
+                                      hi2(n.r_hi_xy), hi2(n.r_z), tminf, boundf);
+                if (il && ir && sp >= st.capacity) {
+                    atomicOr(p.error_word, kErrStackOverflow);
+                    give_up();
+                } else if (il && ir) {
+                    st.put(sp++, n.rptr);
+                    node = n.lptr;
+                } else if (il || ir) {
+                    node = il ? n.lptr : n.rptr;
+                } else {
+                    node = st.get(--sp);
+                }
             }
         }
-        r.flags = AE_HIT_RETESTED | (bi >= 0 ? AE_HIT_HIT : 0u) | (bad ? AE_HIT_OVERFLOW : 0u);
-        r.triPtr = bi;
-        r.t = best;
-        r.t_second = second <= second_limit(best) ? second : INFINITY;
-        p.out[i] = r;
+        const uint32_t waiting = __ballot_sync(kFull, have && waits);
+        if (waiting && (__popc(waiting) >= kRetestBatch || waiting == active) && have && waits) {
+            const double o[3] = { of[0], of[1], of[2] }, d[3] = { df[0], df[1], df[2] };
+            const float4* tq = p.tris + size_t(tp) * 3;
+            const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
+            double t;
+            if (tri64(o, d, A, B, C, bound, t) && t > p.tmin && t < p.tmax &&
+                !(bi >= 0 && t == best && same_triangle(p.tris + size_t(bi) * 3, A, B, C))) {
+                if (t < best || (t == best && tp < bi)) {
+                    if (tp != bi) second = best;
+                    best = t;
+                    bi = tp;
+                } else if (t < second && tp != bi) {
+                    second = t;
+                }
+                // prune by the second distance, and by the window past the nearest
+                // beyond which a second distance is not reported
+                bound = fmin(fmin(p.tmax, second), second_limit(best));
+                boundf = __double2float_ru(bound);
+            }
+            waits = false;
+            if (end) {
+                tp = -1;
+                node = st.get(--sp);
+            } else {
+                tp++;
+            }
+        }
+        if (have && node == kStackEnd && !waits) {
+            ae_hit_f64 r;
+            r.reserved[0] = r.reserved[1] = 0;
+            r.flags = AE_HIT_RETESTED | (bi >= 0 ? AE_HIT_HIT : 0u) | (bad ? AE_HIT_OVERFLOW : 0u);
+            r.triPtr = bi;
+            r.t = best;
+            r.t_second = second <= second_limit(best) ? second : INFINITY;
+            p.out[i] = r;
+            take();
+        }
     }
 }
 
@@ -300,10 +366,11 @@ extern "C" ae_rt_status ae_rt_retest_near_ties(ae_rt_ctx* ctx, int32_t mesh_id, 
     const uint32_t blocks = (n_rays + 255) / 256 < cap ? (n_rays + 255) / 256 : cap;
     retest_compact_kernel<<<blocks, 256, 0, s>>>(p);
     AE_CUDA(ctx, cudaGetLastError());
-    // one listed ray per thread: enough threads for every ray being flagged
-    const uint32_t cap2 = uint32_t(ctx->sm_count) * 16u;
-    const uint32_t blocks2 = (n_rays + 127) / 128 < cap2 ? (n_rays + 127) / 128 : cap2;
-    retest_kernel<<<blocks2, 128, 0, s>>>(p);
+    // every warp of a full GPU: the flagged rays (a few percent) spread over them
+    const uint32_t warps_per_block = kRetestThreads / 32;
+    const uint32_t cap2 = uint32_t(ctx->sm_count) * uint32_t(kRetestBlocks);
+    const uint32_t blocks2 = std::min((n_rays + warps_per_block - 1) / warps_per_block, cap2);
+    retest_kernel<<<blocks2, kRetestThreads, 0, s>>>(p);
     AE_CUDA(ctx, cudaGetLastError());
     if (n_retested) {
         AE_CUDA(ctx, cudaMemcpyAsync(n_retested, p.n_retested, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

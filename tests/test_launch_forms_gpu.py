@@ -113,3 +113,27 @@ def test_transparency_stacks_on_an_opaque_chain(entries):
             assert np.array_equal(vis, 1.0 - occ[:n].astype(np.float32))
     finally:
         c.close()
+
+
+def test_retest_of_any_number_of_rays_gives_the_full_records(ctx):
+    """Near-tie re-tests of one to all of 40,000 rays at mesh edges: the
+    grouping of the double-precision tests does not show in the results."""
+    import torch
+    b = BVH(scenes.terrain_boxes(seed=5, grid=48, n_boxes=6)[0])
+    mid = ctx.upload_mesh(b.nodes, b.pack_triangles())
+    rng = np.random.default_rng(6)
+    n = 40000
+    at = b._verts.reshape(-1, 3)[rng.integers(0, 3 * b.n_input, n)]      # vertices, where triangles tie
+    o = np.array([[50.0, 60.0, -20.0]], np.float32) + rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    d = (at - o).astype(np.float32)
+    rays = torch.from_numpy(scenes.pack_rays(o.astype(np.float32), d / np.linalg.norm(d, axis=1, keepdims=True))).cuda()
+    hits = torch.zeros((n, 8), device="cuda")
+    ctx.trace_closest(mid, rays, 0.0, 1e12, out=hits)
+    full = torch.zeros((n, 8), device="cuda")
+    flagged = ctx.retest_near_ties(mid, rays, hits, 0.0, 1e12, full)
+    assert flagged > n // 4
+    for k in (1, 2, 31, 33, 1000, 2433, 20000):
+        part = torch.zeros((n, 8), device="cuda")
+        ctx.retest_near_ties(mid, rays, hits, 0.0, 1e12, part, n_rays=k)
+        assert torch.equal(part[:k].view(torch.int32), full[:k].view(torch.int32)), k
+        assert not part[k:].any()
