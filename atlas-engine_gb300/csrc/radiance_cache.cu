@@ -36,6 +36,7 @@ struct ae_rc {
     __half* grid_snap = nullptr;
     __nv_bfloat16* mlp_snap = nullptr;
     float* d_loss = nullptr;
+    float* h_loss = nullptr;       // pinned: where the host reads it
     uint32_t* d_counts = nullptr;  // [0] training samples, [1] cache queries
     Scratch samples, queries;
     uint64_t step = 0;
@@ -76,16 +77,19 @@ uint32_t GridBlocks(ae_rc* rc, uint32_t n) {
 }
 
 // Gradients of the relative L2 loss over n training records (device) into
-// mlp_grad / grid_grad (zeroed first); loss sum into d_loss.
+// mlp_grad / grid_grad (zeroed first); loss sum into d_loss.  mlp_out,
+// grid_out: device memory that receives them in place of the cache's buffers.
 ae_rt_status Backprop(ae_rc* rc, const float4* recs, uint32_t n, const uint32_t* n_dev, uint32_t slice,
-                      uint32_t slices, cudaStream_t s) {
-    if (!rc->grads_zero) {
-        RC_CUDA(rc, cudaMemsetAsync(rc->mlp_grad, 0, RC_NPARAM * sizeof(float), s));
-        RC_CUDA(rc, cudaMemsetAsync(rc->grid_grad, 0, rc->grid_params * sizeof(float), s));
-    }
-    rc->grads_zero = false;
+                      uint32_t slices, cudaStream_t s, float* mlp_out = nullptr, float* grid_out = nullptr) {
+    float* mlp = mlp_out ? mlp_out : rc->mlp_grad;
+    float* grid = grid_out ? grid_out : rc->grid_grad;
+    if (mlp_out || !rc->grads_zero) RC_CUDA(rc, cudaMemsetAsync(mlp, 0, RC_NPARAM * sizeof(float), s));
+    if (grid_out || !rc->grads_zero) RC_CUDA(rc, cudaMemsetAsync(grid, 0, rc->grid_params * sizeof(float), s));
+    if (!mlp_out || !grid_out) rc->grads_zero = false;
     RC_CUDA(rc, cudaMemsetAsync(rc->d_loss, 0, sizeof(float), s));
     RcMlpParams p = MlpParams(rc);
+    p.grad_w = mlp;
+    p.grid.grad = reinterpret_cast<float2*>(grid);
     p.recs = recs;
     p.n = n;
     p.n_dev = n_dev;
@@ -97,6 +101,16 @@ ae_rt_status Backprop(ae_rc* rc, const float4* recs, uint32_t n, const uint32_t*
     else
         rc_train_tc_kernel<<<GridBlocks(rc, count), RCTT_THREADS, RCTT_SMEM, s>>>(p);
     RC_CUDA(rc, cudaGetLastError());
+    return AE_RT_OK;
+}
+
+// The loss of the work queued on `s`, waited for: through a pinned word, so
+// that the copy needs no staging.
+ae_rt_status ReadLoss(ae_rc* rc, float* loss_out, cudaStream_t s) {
+    if (!rc->h_loss) RC_CUDA(rc, cudaHostAlloc(&rc->h_loss, sizeof(float), cudaHostAllocDefault));
+    RC_CUDA(rc, cudaMemcpyAsync(rc->h_loss, rc->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+    RC_CUDA(rc, cudaStreamSynchronize(s));
+    *loss_out = *rc->h_loss;
     return AE_RT_OK;
 }
 
@@ -132,6 +146,7 @@ void Destroy(ae_rc* rc) {
                      (void*)rc->grid_grad, (void*)rc->grid_f16, (void*)rc->d_loss, (void*)rc->d_counts,
                      (void*)rc->grid_snap, (void*)rc->mlp_snap })
         cudaFree(p);
+    if (rc->h_loss) cudaFreeHost(rc->h_loss);
     rc->samples.release();
     rc->queries.release();
     for (cudaEvent_t e : rc->ev)
@@ -226,12 +241,7 @@ ae_rt_status TrainSteps(ae_rc* rc, uint32_t n_paths, uint32_t steps, float* loss
         st = AdamStep(rc, s);
         if (st != AE_RT_OK) return st;
     }
-    if (loss_out) {
-        float l = 0.0f;
-        RC_CUDA(rc, cudaMemcpyAsync(&l, rc->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-        RC_CUDA(rc, cudaStreamSynchronize(s));
-        *loss_out = l;
-    }
+    if (loss_out) return ReadLoss(rc, loss_out, s);
     return AE_RT_OK;
 }
 
@@ -366,7 +376,7 @@ ae_rt_status RenderFrame(ae_rc* rc, const ae_camera* cam, uint32_t frame, uint32
             RC_CUDA(rc, cudaStreamWaitEvent(a0, rc->ev[0], 0));
             RcMlpParams m0 = mp;
             m0.n_dev = rc->d_counts + 2;
-            rc_infer_tc_kernel<RC_INFER><<<GridBlocks(rc, cap) * 3, RCT_THREADS, RCT_SMEM, a0>>>(m0);
+            rc_infer_tc_kernel<RC_INFER><<<GridBlocks(rc, cap) * RCT_CTAS, RCT_THREADS, RCT_SMEM, a0>>>(m0);
             RC_CUDA(rc, cudaGetLastError());
             RC_CUDA(rc, cudaEventRecord(rc->ev[1], a0));
         }
@@ -375,7 +385,7 @@ ae_rt_status RenderFrame(ae_rc* rc, const ae_camera* cam, uint32_t frame, uint32
     RcMlpParams m1 = mp;
     m1.n_dev = rc->d_counts + 1;
     m1.offset_dev = rc->d_counts + 2;
-    rc_infer_tc_kernel<RC_INFER><<<GridBlocks(rc, cap) * 3, RCT_THREADS, RCT_SMEM, s>>>(m1);
+    rc_infer_tc_kernel<RC_INFER><<<GridBlocks(rc, cap) * RCT_CTAS, RCT_THREADS, RCT_SMEM, s>>>(m1);
     RC_CUDA(rc, cudaGetLastError());
     RC_CUDA(rc, cudaStreamWaitEvent(s, rc->ev[1], 0));
     for (int q = 0; q < 2; q++)
@@ -509,7 +519,7 @@ ae_rt_status ae_rc_predict(ae_rc* rc, const float* queries, uint32_t n, float* o
     p.recs = reinterpret_cast<const float4*>(queries);
     p.n = n;
     p.out = reinterpret_cast<float4*>(out);
-    rc_infer_tc_kernel<RC_PREDICT><<<GridBlocks(rc, n) * 3, RCT_THREADS, RCT_SMEM, static_cast<cudaStream_t>(stream)>>>(p);
+    rc_infer_tc_kernel<RC_PREDICT><<<GridBlocks(rc, n) * RCT_CTAS, RCT_THREADS, RCT_SMEM, static_cast<cudaStream_t>(stream)>>>(p);
     RC_CUDA(rc, cudaGetLastError());
     return AE_RT_OK;
 }
@@ -546,17 +556,19 @@ ae_rt_status ae_rc_gradients(ae_rc* rc, const float* samples, uint32_t n, float*
     if (n == 0 || !DevPtr(samples)) return RcFail(rc, AE_RT_INVALID_ARG, "ae_rc_gradients takes device samples");
     RC_CUDA(rc, cudaSetDevice(rc->ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    ae_rt_status st = Backprop(rc, reinterpret_cast<const float4*>(samples), n, nullptr, 0, 0, s);
+    // into the caller's device buffers at once where their alignment lets the
+    // kernel add in 16 bytes (through the cache's own, 2 x 67 MB of copy at 2^19
+    // entries a level)
+    auto direct = [](float* g) { return g && DevPtr(g) && (reinterpret_cast<uintptr_t>(g) & 15u) == 0 ? g : nullptr; };
+    float* const mlp_out = direct(grad_mlp);
+    float* const grid_out = direct(grad_grid);
+    ae_rt_status st = Backprop(rc, reinterpret_cast<const float4*>(samples), n, nullptr, 0, 0, s, mlp_out, grid_out);
     if (st != AE_RT_OK) return st;
-    if (grad_mlp) RC_CUDA(rc, cudaMemcpyAsync(grad_mlp, rc->mlp_grad, RC_NPARAM * sizeof(float), cudaMemcpyDefault, s));
-    if (grad_grid)
+    if (grad_mlp && !mlp_out)
+        RC_CUDA(rc, cudaMemcpyAsync(grad_mlp, rc->mlp_grad, RC_NPARAM * sizeof(float), cudaMemcpyDefault, s));
+    if (grad_grid && !grid_out)
         RC_CUDA(rc, cudaMemcpyAsync(grad_grid, rc->grid_grad, rc->grid_params * sizeof(float), cudaMemcpyDefault, s));
-    if (loss_out) {
-        float l = 0.0f;
-        RC_CUDA(rc, cudaMemcpyAsync(&l, rc->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-        RC_CUDA(rc, cudaStreamSynchronize(s));
-        *loss_out = l;
-    }
+    if (loss_out) return ReadLoss(rc, loss_out, s);
     return AE_RT_OK;
 }
 
@@ -569,12 +581,7 @@ ae_rt_status ae_rc_train_batch(ae_rc* rc, const float* samples, uint32_t n, floa
     if (st != AE_RT_OK) return st;
     st = AdamStep(rc, s);
     if (st != AE_RT_OK) return st;
-    if (loss_out) {
-        float l = 0.0f;
-        RC_CUDA(rc, cudaMemcpyAsync(&l, rc->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-        RC_CUDA(rc, cudaStreamSynchronize(s));
-        *loss_out = l;
-    }
+    if (loss_out) return ReadLoss(rc, loss_out, s);
     return AE_RT_OK;
 }
 
@@ -639,12 +646,7 @@ ae_rt_status ae_rc_frame(ae_rc* rc, const ae_camera* cam, uint32_t frame, uint32
     st = RenderFrame(rc, cam, frame, last_bounce, accum, s, true);
     if (st != AE_RT_OK) return st;
     RC_CUDA(rc, cudaStreamWaitEvent(s, rc->ev[3], 0));
-    if (loss_out) {
-        float l = 0.0f;
-        RC_CUDA(rc, cudaMemcpyAsync(&l, rc->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-        RC_CUDA(rc, cudaStreamSynchronize(s));
-        *loss_out = l;
-    }
+    if (loss_out) return ReadLoss(rc, loss_out, s);
     return AE_RT_OK;
 }
 

@@ -3,15 +3,18 @@
 // a tcgen05.mma (M = 128 queries, N = 64 or 16, K = 64 in four K = 16 steps)
 // accumulating in FP32 tensor memory.
 //
-// Per CTA (two independent groups of 128 threads, one query row per thread;
-// 3 CTAs per SM), per group:
+// Per CTA (three independent groups of 128 threads, one query row per thread;
+// 2 CTAs per SM: the same six groups as three CTAs of two, with one copy of
+// the weights less in shared memory, which the L1 cache of the hash-grid
+// gathers gets: 92 against 116 us for 500,001 queries; seven groups in one CTA
+// take 96, four 101, eight 113), per group:
 //  * shared memory holds the weights of all six layers (shared by the
 //    groups) and the group's 128 x 64 BF16 activation tile, both in the
 //    no-swizzle core-matrix layout the MMA
 //    descriptors describe: 8 rows x 16 bytes per core matrix, core matrices
 //    128 bytes apart along K (leading byte offset) and 1024 bytes apart along
 //    M / N (stride byte offset);
-//  * warp 0 allocates 128 tensor-memory columns, 64 per group (lane i =
+//  * warp 0 allocates 256 tensor-memory columns, 64 per group (lane i =
 //    query row i of the group's tile);
 //  * per layer thread 0 issues the four MMAs and commits them to an
 //    mbarrier; every thread waits on it (bounded by the global timer), reads
@@ -39,10 +42,11 @@ constexpr uint32_t RCT_SBO = 1024;                      // core matrices along M
 constexpr uint32_t RCT_ABYTES = RC_TILE * RC_W * 2;     // 16 KB activation tile
 constexpr uint32_t RCT_WLAYER = RC_W * RC_W * 2;        // 8 KB per hidden layer
 constexpr uint32_t RCT_WBYTES = RC_HIDDEN * RCT_WLAYER + RC_OUT * RC_W * 2;   // 43,008
-constexpr uint32_t RCT_GROUPS = 2;                      // independent 128-row tile groups per CTA
+constexpr uint32_t RCT_GROUPS = 3;                      // independent 128-row tile groups per CTA
+constexpr uint32_t RCT_CTAS = 2;                        // CTAs an SM
 constexpr uint32_t RCT_THREADS = RCT_GROUPS * RC_TILE;
 constexpr uint32_t RCT_SMEM = RCT_WBYTES + RCT_GROUPS * RCT_ABYTES + 64;      // + mbarriers, flags, TMEM address
-constexpr uint32_t RCT_TMEM_COLS = RCT_GROUPS * 64;
+constexpr uint32_t RCT_TMEM_COLS = 256;                 // 64 per group, a power of two
 
 // Byte offset of the 16-byte chunk (row, k-block kb) in the blocked layout.
 __device__ __forceinline__ uint32_t rct_off(uint32_t row, uint32_t kb) {
@@ -85,9 +89,11 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 
 // Waits for the mbarrier phase with parity `parity`; false after ~200 ms of
-// the global timer, or after 2^25 polls whatever the timer says.
+// the global timer, or after 2^25 polls whatever the timer says.  The timer
+// is first read after 64 polls without success: a read of it at every wait
+// is slow next to the waits themselves.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    const uint64_t start = global_ns();
+    uint64_t start = 0;
     for (uint32_t it = 0; it < (1u << 25); it++) {
         uint32_t done;
         asm volatile(
@@ -95,24 +101,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
         if (done) return true;
-        if ((it & 63u) == 63u && global_ns() - start > 200000000ull) return false;
+        if ((it & 63u) == 63u) {
+            const uint64_t now = global_ns();
+            if (it == 63u) start = now;
+            else if (now - start > 200000000ull) return false;
+        }
     }
     return false;
 }
 
 // Barrier of one 128-thread tile group (named barrier 1 + group).
 __device__ __forceinline__ void group_sync(uint32_t g) {
-    static_assert(RCT_GROUPS == 2, "one named barrier per group");
-    if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-    else asm volatile("bar.sync 2, 128;" ::: "memory");
+    asm volatile("bar.sync %0, 128;" :: "r"(g + 1u) : "memory");
 }
 
-// rc_encode_values with four levels' table reads in flight at once.
+// rc_encode_values with all levels unrolled: many table reads in flight, and
+// the encoded values in registers (a partly unrolled loop indexed them in
+// local memory: 155 against 116 us for 500,001 queries).
 __device__ __forceinline__ void rc_encode_values_wide(const RcGrid& g, const float4& q0, const float4& q1,
                                                       const float4& q2, __nv_bfloat162 v[32]) {
     float x[3];
     rc_unit(g, q0, x);
-#pragma unroll 4
+#pragma unroll
     for (int l = 0; l < RC_LEVELS; l++) {
         uint32_t idx[8];
         float w[8];
@@ -138,6 +148,105 @@ __device__ __forceinline__ void rc_encode_values_wide(const RcGrid& g, const flo
     for (int k = 27; k < 32; k++) v[k] = __floats2bfloat162_rn(0.0f, 0.0f);
 }
 
+// Grid levels l0 .. l0 + 3 of one record: the 16-byte chunk l0 / 4 of its row.
+__device__ __forceinline__ uint4 rc_encode_levels(const RcGrid& g, const float4& q0, uint32_t l0) {
+    float x[3];
+    rc_unit(g, q0, x);
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int l = int(l0) + j;
+        uint32_t idx[8];
+        float w[8];
+        rc_corners(g, l, x, idx, w);
+        float a0 = 0.0f, a1 = 0.0f;
+        const __half2* tab = g.table + size_t(l) * g.T;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float2 e = __half22float2(tab[idx[k]]);
+            a0 += w[k] * e.x;
+            a1 += w[k] * e.y;
+        }
+        v[j] = pack_bf16(a0, a1);
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+// Adds one record's gradients of a level's eight corners.  Corners 2j and
+// 2j + 1 differ in x alone: where their entries are the two of one aligned
+// pair, one 16-byte addition takes both.
+__device__ __forceinline__ void rc_add_corners(float2* gt, const uint32_t idx[8], const float2 v[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        if (idx[k + 1] == (idx[k] ^ 1u)) {
+            const bool odd = idx[k] & 1u;
+            const float2 lo = odd ? v[k + 1] : v[k], hi = odd ? v[k] : v[k + 1];
+            atomicAdd(reinterpret_cast<float4*>(gt + (idx[k] & ~1u)), make_float4(lo.x, lo.y, hi.x, hi.y));
+        } else {
+            atomicAdd(&gt[idx[k]], v[k]);
+            atomicAdd(&gt[idx[k + 1]], v[k + 1]);
+        }
+    }
+}
+
+// Their gradient (4 pairs of BF16, zero for a lane without a record)
+// scattered to the table; the whole warp calls it.  Neighbouring records
+// often lie in one cell of the coarse levels: runs of lanes with the same cell
+// are summed by shuffles first and added once.  The additions, not the tensor
+// cores, are what a tile waits for, and each costs its lane's own pass
+// through the memory pipeline.  A gradient call of 65,536 records in image
+// order: 196 us with one addition per corner and record by one thread a
+// record, 178 by four, 125 with runs summed and pairs added together (168
+// without the runs), 120 with the weight gradients spread over the layers and
+// added in 16 bytes.
+constexpr int kRunLanes = 8;            // lanes in a run behind its first before runs are summed
+__device__ __forceinline__ void rc_scatter_levels(const RcGrid& g, const float4& q0, uint32_t l0, const uint4& d) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, upto = (2u << lane) - 1u;      // lanes 0 .. lane
+    float x[3];
+    rc_unit(g, q0, x);
+    const uint32_t dv[4] = { d.x, d.y, d.z, d.w };
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint32_t bits = j == 0 ? dv[0] : j == 1 ? dv[1] : j == 2 ? dv[2] : dv[3];
+        const float2 gr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bits));
+        const int l = int(l0) + j;
+        uint32_t idx[8];
+        float w[8];
+        rc_corners(g, l, x, idx, w);
+        float2 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = make_float2(w[k] * gr.x, w[k] * gr.y);
+        float2* gt = g.grad + size_t(l) * g.T;
+        bool adds = gr.x != 0.0f || gr.y != 0.0f;
+        // eight equal corners: the same entries, whatever the cell
+        bool same = lane != 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) same = (__shfl_up_sync(kFull, idx[k], 1) == idx[k]) && same;
+        const uint32_t sames = __ballot_sync(kFull, same);
+        if (__popc(sames) >= kRunLanes) {
+            const uint32_t after = ~sames & ~upto;                  // first lanes of later runs
+            const uint32_t tail = after ? __ffs(after) - 2u : 31u;  // last lane of this run
+            uint32_t longer = sames;                                // bit i: lanes i .. i + off - 1 all continue a run
+#pragma unroll 1
+            for (uint32_t off = 1; longer; off <<= 1) {
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float ox = __shfl_down_sync(kFull, v[k].x, off), oy = __shfl_down_sync(kFull, v[k].y, off);
+                    if (lane + off <= tail) { v[k].x += ox; v[k].y += oy; }
+                }
+                longer &= longer >> off;
+            }
+            adds = !same;
+        }
+        if (adds) rc_add_corners(gt, idx, v);
+    }
+}
+
+__device__ __forceinline__ uint4 pack_bf16x8(const float* v) {
+    return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+
 // 16 consecutive FP32 columns of this thread's tensor-memory lane.
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float v[16]) {
     uint32_t r[16];
@@ -153,7 +262,7 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float v[16]) {
 }
 
 template <int MODE>
-static __global__ void __launch_bounds__(RCT_THREADS) rc_infer_tc_kernel(RcMlpParams p) {
+static __global__ void __launch_bounds__(RCT_THREADS, RCT_CTAS) rc_infer_tc_kernel(RcMlpParams p) {
     extern __shared__ __align__(1024) unsigned char rct_smem[];
     unsigned char* wsm = rct_smem;
     unsigned char* tail = rct_smem + RCT_WBYTES + RCT_GROUPS * RCT_ABYTES;
@@ -284,7 +393,9 @@ static __global__ void __launch_bounds__(RCT_THREADS) rc_infer_tc_kernel(RcMlpPa
 //  * the MMA group (warps 0-3, one record row per thread) issues the MMAs,
 //    reads the accumulators back, applies ReLU / the loss / the ReLU
 //    derivative and writes the next operand tile;
-//  * the producer group (warps 4-7) encodes tile k + 1's records (the
+//  * the producer group (warps 4-19, four threads a record; with one thread a
+//    record its chains of gathers and additions were the longer half of a
+//    tile) encodes tile k + 1's records (the
 //    hash-grid gathers) into the other of two input tiles while the MMA group
 //    works on tile k, and scatters the hash-grid gradient of tile k - 1 (the
 //    atomics) from a staging buffer the MMA group fills at the end of a tile.
@@ -318,10 +429,11 @@ constexpr uint32_t RCTT_A0 = 44032;                                      // 2 in
 constexpr uint32_t RCTT_AH = RCTT_A0 + 2 * RCT_ABYTES;                   // hidden activations A_1 .. A_5
 constexpr uint32_t RCTT_DZ = RCTT_AH + RC_HIDDEN * RCT_ABYTES;           // dP / dZ tile
 constexpr uint32_t RCTT_DG = RCTT_DZ + RCT_ABYTES + 2048;                // + margin; 2 x 128 grid-gradient rows (64 B)
-constexpr uint32_t RCTT_Q0 = RCTT_DG + 2 * RC_TILE * 64;                 // 2 x 128 record positions (float4)
-constexpr uint32_t RCTT_TAIL = RCTT_Q0 + 2 * RC_TILE * 16;               // mbarriers, flag, tensor-memory address
+constexpr uint32_t RCTT_TAIL = RCTT_DG + 2 * RC_TILE * 64;               // mbarriers, flag, tensor-memory address
 constexpr uint32_t RCTT_SMEM = RCTT_TAIL + 64;
-constexpr uint32_t RCTT_THREADS = 2 * RC_TILE;
+constexpr uint32_t RCTT_PARTS = 4;                                       // producer threads per record, 4 levels each
+constexpr uint32_t RCTT_PRODUCERS = RCTT_PARTS * RC_TILE;
+constexpr uint32_t RCTT_THREADS = RC_TILE + RCTT_PRODUCERS;
 constexpr uint32_t RCTT_TMEM_COLS = 512;
 constexpr uint32_t RCTT_DW = 64;                                         // first weight-gradient column
 
@@ -365,7 +477,8 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&bars[0])) : "memory");
         for (int b = 1; b < 5; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&bars[b])), "r"(RC_TILE) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;"
+                         :: "r"(smem_u32(&bars[b])), "r"(b < 3 ? RCTT_PRODUCERS : uint32_t(RC_TILE)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0u;
     }
@@ -550,7 +663,9 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
         if (ok && accw && warp < 2) {
             const uint32_t out = row;       // warps 0 and 1: lanes 0-63
 #pragma unroll 1
-            for (int l = 0; l <= RC_HIDDEN; l++) {
+            for (uint32_t i = 0; i <= uint32_t(RC_HIDDEN); i++) {
+                // the CTAs arrive together: each starts with another layer
+                const int l = int((i + blockIdx.x) % uint32_t(RC_HIDDEN + 1));
                 float g[64];
 #pragma unroll
                 for (uint32_t c = 0; c < 4; c++)
@@ -559,14 +674,18 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
                 if (out < nout) {
                     float* gw = p.grad_w + size_t(l) * RC_W * RC_W + size_t(out) * RC_W;
 #pragma unroll
-                    for (int j = 0; j < 64; j += 2)
-                        atomicAdd(reinterpret_cast<float2*>(gw + j), make_float2(g[j], g[j + 1]));
+                    for (int j = 0; j < 64; j += 4)
+                        atomicAdd(reinterpret_cast<float4*>(gw + j), make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]));
                 }
             }
         }
     } else {
         // producer: encode tile k into input tile k & 1 after scattering the
-        // gradient of tile k - 2, staged in the same buffer; then the last two
+        // gradient of tile k - 2, staged in the same buffer; then the last two.
+        // Four threads share a record: thread `part` takes levels 4 part to
+        // 4 part + 3, which are 16-byte chunk `part` of the input row, and
+        // chunk 4 + part of its other inputs.
+        const uint32_t part = (tid - RC_TILE) / RC_TILE;
 #pragma unroll 1
         for (uint32_t k = 0; k < my_tiles + 2 && ok; k++) {
             const uint32_t b = k & 1u;
@@ -574,29 +693,33 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
                 const uint32_t kk = k - 2;
                 if (!mbar_wait(grads_bar(b), (kk >> 1) & 1u)) { *fail = 1u; ok = false; break; }
                 const uint32_t gi = (blockIdx.x + kk * gridDim.x) * RC_TILE + row;
-                if (gi < count) {
-                    const float4 q0 = reinterpret_cast<const float4*>(rctt_smem + RCTT_Q0)[b * RC_TILE + row];
-                    rc_encode_backward(p.grid, q0, reinterpret_cast<const __nv_bfloat16*>(
-                                                       rctt_smem + RCTT_DG + (b * RC_TILE + row) * 64u));
-                }
+                const bool valid = gi < count;
+                const float4 q0 = valid ? p.recs[size_t(first + gi) * 4] : make_float4(0, 0, 0, 0);
+                const uint4 dg = valid ? reinterpret_cast<const uint4*>(rctt_smem + RCTT_DG +
+                                                                        (b * RC_TILE + row) * 64u)[part]
+                                       : make_uint4(0, 0, 0, 0);
+                rc_scatter_levels(p.grid, q0, part * 4u, dg);
             }
             if (k < my_tiles) {
                 const uint32_t gi = (blockIdx.x + k * gridDim.x) * RC_TILE + row;
-                __nv_bfloat162 v[32];
-                float4 q0 = make_float4(0, 0, 0, 0);
+                uint4 lv = make_uint4(0, 0, 0, 0), other = lv;
                 if (gi < count) {
                     const float4* rec = p.recs + size_t(first + gi) * 4;
-                    q0 = rec[0];
-                    rc_encode_values_wide(p.grid, q0, rec[1], rec[2], v);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = __floats2bfloat162_rn(0.0f, 0.0f);
+                    const float4 q0 = rec[0];
+                    lv = rc_encode_levels(p.grid, q0, part * 4u);
+                    if (part < 2) {
+                        const float4 q1 = rec[1];
+                        float sh[16];
+                        sh16(q1.x, q1.y, q1.z, sh);
+                        other = part == 0 ? pack_bf16x8(sh) : pack_bf16x8(sh + 8);
+                    } else if (part == 2) {
+                        const float4 q2 = rec[2];
+                        other = make_uint4(pack_bf16(q2.x, q2.y), pack_bf16(q2.z, q0.w), pack_bf16(q2.w, 0.0f), 0u);
+                    }
                 }
                 unsigned char* a0 = act_ptr(0, b);
-#pragma unroll
-                for (uint32_t kb = 0; kb < 8; kb++)
-                    *reinterpret_cast<uint4*>(a0 + rct_off(row, kb)) = reinterpret_cast<const uint4*>(v)[kb];
-                reinterpret_cast<float4*>(rctt_smem + RCTT_Q0)[b * RC_TILE + row] = q0;
+                *reinterpret_cast<uint4*>(a0 + rct_off(row, part)) = lv;
+                *reinterpret_cast<uint4*>(a0 + rct_off(row, 4u + part)) = other;
                 proxy_fence();
                 mbar_arrive(full_bar(b));
             }
