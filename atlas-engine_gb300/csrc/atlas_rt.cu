@@ -260,11 +260,13 @@ namespace {
 
 // depth: stack entries the launch's trees can need (batched launches hold
 // kStackEntries at most and report overflow beyond).
+// p.work_counter: a word that an earlier kernel on `s` zeroed, or null (one of
+// the context's).
 // camera: the rays are p.cam's camera rays (single mesh, closest hit, a tree
 // within kStackEntries, exact, no counters: Trace checks this).
 ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStream_t s, bool ties, uint32_t depth,
                     bool camera = false) {
-    AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
+    if (!p.work_counter) AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
@@ -300,7 +302,7 @@ atlas::rt::dev::CameraParams CameraFrom(const ae_camera* cam) {
 ae_rt_status Trace(ae_rt_ctx* ctx, bool any, int32_t mesh_id, const ae_packed_ray* rays, uint32_t n_rays,
                    float tmin, float tmax, void* out, void* stream, const uint32_t* count_dev = nullptr,
                    uint32_t cull_mask = 0xffffffffu, bool per_ray_tmax = false, bool ties = true,
-                   const atlas::rt::dev::CameraParams* cam = nullptr) {
+                   const atlas::rt::dev::CameraParams* cam = nullptr, uint32_t* counter = nullptr) {
     if (!ctx) return AE_RT_INVALID_ARG;
     const bool scene = mesh_id == kSceneTarget;
     if (scene && !ctx->scene_ready) return Fail(ctx, AE_RT_INVALID_ARG, "no scene has been set");
@@ -367,6 +369,7 @@ ae_rt_status Trace(ae_rt_ctx* ctx, bool any, int32_t mesh_id, const ae_packed_ra
     }
     p.per_ray_tmax = per_ray_tmax ? 1u : 0u;
     if (camera) p.cam = *cam;
+    p.work_counter = counter;
     ae_rt_status st = Launch(ctx, any, scene ? MODE_SCENE : MODE_MESH, p, s, ties, scene ? ctx->scene_depth : m.depth,
                              camera);
     if (st != AE_RT_OK) return st;
@@ -524,7 +527,7 @@ void ae_rt_ctx_destroy(ae_rt_ctx* ctx) {
     for (Scratch* sc : { &ctx->pt_rays[0], &ctx->pt_rays[1], &ctx->pt_pay[0], &ctx->pt_pay[1], &ctx->pt_hits,
                          &ctx->pt_shadow, &ctx->pt_shadow_pay, &ctx->pt_occ, &ctx->pt_shadow2, &ctx->pt_shadow_pay2,
                          &ctx->pt_occ2, &ctx->pass_rays, &ctx->pass_key, &ctx->pass_hits, &ctx->pass_rad,
-                         &ctx->pass_shadow, &ctx->pass_shadow_pay, &ctx->pass_vis, &ctx->pass_counts })
+                         &ctx->pass_shadow, &ctx->pass_shadow_pay, &ctx->pass_vis, &ctx->pass_counts, &ctx->pt_words })
         sc->release();
     for (cudaEvent_t e : ctx->pt_events)
         if (e) cudaEventDestroy(e);
@@ -1173,6 +1176,15 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
     }
     // every queue holds at most one ray per pixel of the tile
     const uint32_t blocks = (n_tile + 255) / 256;
+    const uint32_t shade_blocks = (n_tile + atlas::rt::dev::kShadeThreads - 1) / atlas::rt::dev::kShadeThreads;
+    // counters of one sample, set by its ray generation: per bounce the queue's
+    // length, its shadow queue's and the work counters of the two traces (a
+    // memset for each was a stream operation of its own)
+    // (past kWordSets bounces the sets are used again, cleared one bounce ahead)
+    constexpr uint32_t kWordSets = 1024;
+    p.n_words = 4 * uint32_t(std::min<uint64_t>(uint64_t(params->max_bounces) + 2, kWordSets));
+    AE_CUDA(ctx, ctx->pt_words.ensure(p.n_words * sizeof(uint32_t)));
+    p.words = static_cast<uint32_t*>(ctx->pt_words.ptr);
     const float kInf = 1e12f;   // INF of common.hsh:8
     // Shadow queues alternate between two buffers: a bounce's shadow trace and
     // resolve run on the side stream while the next bounce is traced and shaded
@@ -1187,10 +1199,9 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
     for (uint32_t smp = 0; smp < params->spp; smp++) {
         p.sample = params->sample_offset + smp;
         p.gb_write = (smp == 0 && p.gb_mats) ? 1u : 0u;
-        // ray generation into queue 0
+        // ray generation into queue 0; it also sets the sample's counters
         p.rays_out = static_cast<float4*>(ctx->pt_rays[0].ptr);
         p.pay_out = static_cast<float4*>(ctx->pt_pay[0].ptr);
-        p.n_out = ctx->d_pt_counts + 0;
         atlas::rt::dev::pt_raygen_kernel<<<blocks, 256, 0, s>>>(c, p);
         AE_CUDA(ctx, cudaGetLastError());
         for (uint32_t b = 0; b <= params->max_bounces; b++) {
@@ -1198,26 +1209,27 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
             p.bounce = b;
             p.rays_in = static_cast<const float4*>(ctx->pt_rays[in].ptr);
             p.pay_in = static_cast<const float4*>(ctx->pt_pay[in].ptr);
-            p.n_in = ctx->d_pt_counts + in;
+            uint32_t* const w = p.words + 4 * size_t(b % kWordSets);
+            uint32_t* const next = p.words + 4 * size_t((b + 1) % kWordSets);
+            if (b + 1 >= kWordSets) AE_CUDA(ctx, cudaMemsetAsync(next, 0, 4 * sizeof(uint32_t), s));
+            p.n_in = w;
             p.rays_out = static_cast<float4*>(ctx->pt_rays[out].ptr);
             p.pay_out = static_cast<float4*>(ctx->pt_pay[out].ptr);
-            p.n_out = ctx->d_pt_counts + out;
+            p.n_out = next;
             p.shadow_rays = static_cast<float4*>(shadowRays[q]->ptr);
             p.shadow_pay = static_cast<float4*>(shadowPay[q]->ptr);
-            p.n_shadow = ctx->d_pt_counts + 2 + q;
+            p.n_shadow = w + 1;
             p.shadow_occ = static_cast<const uint8_t*>(shadowOcc[q]->ptr);
             const ae_packed_ray* rays_in = static_cast<const ae_packed_ray*>(ctx->pt_rays[in].ptr);
             ae_rt_status st = transparent
                 ? TraceTransparency(ctx, false, rays_in, n, 0.0f, kInf, AE_RT_MASK_ALL, ctx->pt_hits.ptr, stream,
-                                    ctx->d_pt_counts + in)
+                                    p.n_in, false, w + 2)
                 : Trace(ctx, false, kSceneTarget, rays_in, n, 0.0f, kInf, ctx->pt_hits.ptr, stream,
-                        ctx->d_pt_counts + in, AE_RT_MASK_ALL, false, false);
+                        p.n_in, AE_RT_MASK_ALL, false, false, nullptr, w + 2);
             if (st != AE_RT_OK) return st;
             // this shadow queue's previous resolve must be done before it is refilled
             if (pending[q]) AE_CUDA(ctx, cudaStreamWaitEvent(s, ctx->pt_events[2 + q], 0));
-            AE_CUDA(ctx, cudaMemsetAsync(ctx->d_pt_counts + out, 0, sizeof(uint32_t), s));
-            AE_CUDA(ctx, cudaMemsetAsync(p.n_shadow, 0, sizeof(uint32_t), s));
-            atlas::rt::dev::pt_shade_kernel<<<blocks, 256, 0, s>>>(p);
+            atlas::rt::dev::pt_shade_kernel<<<shade_blocks, atlas::rt::dev::kShadeThreads, 0, s>>>(p);
             AE_CUDA(ctx, cudaGetLastError());
             AE_CUDA(ctx, cudaEventRecord(ctx->pt_events[q], s));
             AE_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pt_events[q], 0));
@@ -1226,11 +1238,11 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
                 AE_CUDA(ctx, ctx->pt_vis[q].ensure(size_t(n) * sizeof(float)));
                 p.shadow_vis = static_cast<const float*>(ctx->pt_vis[q].ptr);
                 st = TraceTransparency(ctx, true, shadow_in, n, 0.0f, kInf, AE_RT_MASK_SHADOW, ctx->pt_vis[q].ptr, side,
-                                       p.n_shadow, true);
+                                       p.n_shadow, true, w + 3);
             } else {
                 p.shadow_vis = nullptr;
                 st = Trace(ctx, true, kSceneTarget, shadow_in, n, 0.0f, kInf, shadowOcc[q]->ptr, side, p.n_shadow,
-                           AE_RT_MASK_SHADOW, true);
+                           AE_RT_MASK_SHADOW, true, true, nullptr, w + 3);
             }
             if (st != AE_RT_OK) return st;
             atlas::rt::dev::pt_resolve_kernel<<<blocks, 256, 0, side>>>(p);

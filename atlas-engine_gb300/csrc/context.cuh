@@ -102,6 +102,7 @@ struct ae_rt_ctx {
     float env[3] = { 0.0f, 0.0f, 0.0f };  // constant environment radiance of the path tracer's misses
     // path tracer queues
     atlas::rt::host::Scratch pt_rays[2], pt_pay[2], pt_hits, pt_shadow, pt_shadow_pay, pt_occ;
+    atlas::rt::host::Scratch pt_words;  // per-bounce counters of a sample
     atlas::rt::host::Scratch pt_gb;     // real-time G-buffer matrices
     atlas::rt::host::Scratch pt_vis[2]; // shadow visibility of the transparency traversal, per shadow queue
     // a second shadow queue: a bounce's shadow trace runs beside the next bounce's trace
@@ -110,7 +111,7 @@ struct ae_rt_ctx {
     // scratch of the RTAO / reflection / GI / DDGI passes (consumers.cu)
     atlas::rt::host::Scratch pass_rays, pass_key, pass_hits, pass_rad, pass_shadow, pass_shadow_pay, pass_vis,
         pass_counts;
-    uint32_t* d_pt_counts = nullptr;    // [0], [1] ray queues, [2], [3] shadow queues
+    uint32_t* d_pt_counts = nullptr;    // radiance-cache render: [0], [1] ray queues, [2], [3] shadow queues
     uint32_t* d_counter = nullptr;     // [1] error word; [0], [2..6] work counters (rotated per launch)
     uint32_t next_work_slot = 0;
     unsigned long long* d_fetch = nullptr;
@@ -182,10 +183,12 @@ ae_rt_status TraceSceneQueue(ae_rt_ctx* ctx, bool any, const ae_packed_ray* rays
 
 // The transparency traversal variants over the scene (transparency.cu); with
 // count_dev, `n` is the queue capacity and the count lives on the device;
-// with per_ray_tmax, ray i's tmax is its third vector's x.
+// with per_ray_tmax, ray i's tmax is its third vector's x; counter: a work
+// counter that an earlier kernel on the stream zeroed, or null.
 ae_rt_status TraceTransparency(ae_rt_ctx* ctx, bool any, const ae_packed_ray* rays, uint32_t n, float tmin,
                                float tmax, uint32_t cull_mask, void* out, void* stream,
-                               const uint32_t* count_dev = nullptr, bool per_ray_tmax = false);
+                               const uint32_t* count_dev = nullptr, bool per_ray_tmax = false,
+                               uint32_t* counter = nullptr);
 
 // The bounce loop's queues for `capacity` rays: two ray/payload queues, the
 // hit buffer, two shadow queues (a bounce's shadow trace runs on

@@ -69,6 +69,8 @@ struct PtParams {
     float4* rays_out;
     float4* pay_out;
     uint32_t* n_out;
+    uint32_t* words;              // ray generation: the sample's n_words counters, or null (n_out alone)
+    uint32_t n_words;
     float4* shadow_rays;
     float4* shadow_pay;           // contribution.rgb, pixel bits
     uint32_t* n_shadow;
@@ -367,7 +369,13 @@ static __global__ void pt_raygen_kernel(CameraParams c, PtParams p) {
     r[1] = make_float4(d.x, d.y, d.z, 0.0f);
     r[2] = make_float4(0.0f, __int_as_float(-1), __int_as_float(-1), 0.0f);
     p.pay_out[i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(pix));
-    if (i == 0) *p.n_out = n;
+    if (p.words) {
+        // the sample's counters: this queue's length, zeros for everything after it
+        if (blockIdx.x == 0)
+            for (uint32_t k = threadIdx.x; k < p.n_words; k += blockDim.x) p.words[k] = k == 0 ? n : 0u;
+    } else if (i == 0) {
+        *p.n_out = n;
+    }
 }
 
 __device__ __forceinline__ void add_radiance(const PtParams& p, uint32_t key, V3 L) {
@@ -782,28 +790,64 @@ __device__ __forceinline__ void write_gbuffer(const PtParams& p, uint32_t pix, b
     }
 }
 
-static __global__ void pt_shade_kernel(PtParams p) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// Threads of pt_shade_kernel's blocks; 6 blocks an SM, 80 registers (256
+// threads without a register bound, 16 warps an SM: 1,336 against 1,303 us for
+// a sample at 1920 x 1080).
+constexpr uint32_t kShadeThreads = 128;
+
+// The block's hits are packed to its front before they are shaded: after the
+// first bounce about half of the rays miss, here and there, and a warp shaded
+// 10 of 32 lanes (22 packed: the second bounce's shading 126 -> 116 us, the
+// third's 46 -> 39, the fourth's 25 -> 18).
+static __global__ void __launch_bounds__(kShadeThreads, 6) pt_shade_kernel(PtParams p) {
+    __shared__ uint32_t s_hits[kShadeThreads / 32 + 1];
+    __shared__ uint8_t s_slot[kShadeThreads];
     const uint32_t n = min(*p.n_in, queue_capacity(p));
+    const uint32_t first = blockIdx.x * kShadeThreads;
+    if (first >= n) return;
     bool emitRay = false, emitShadow = false;
     float4 outRay0{}, outRay1{}, outPay{}, shRay0{}, shRay1{}, shPay{};
-    if (i < n) {
+    const bool gbuffer = p.gb_write && p.bounce == 0;
+    uint32_t hits;
+    {
+        const uint32_t i = first + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        const bool hit = i < n && __float_as_int(p.hits_in[size_t(i) * 2].y) >= 0;
+        if (i < n && !hit) {
+            const float4 pay = p.pay_in[i];
+            const uint32_t pix = __float_as_uint(pay.w);
+            const V3 thr = v3(pay.x, pay.y, pay.z);
+            if (gbuffer) {
+                const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
+                write_gbuffer(p, pix & kPixelMask, false, ld3(o4) + ld3(d4) * 100.0f, v3(1.0f, 0.0f, 0.0f), 0, 0);
+            }
+            // EvaluateBounce's miss: the environment times the throughput, clamped per channel
+            if (p.sc.env_r + p.sc.env_g + p.sc.env_b > 0.0f)
+                add_radiance(p, pix, v3(fminf(p.sc.env_r * thr.x, 10.0f), fminf(p.sc.env_g * thr.y, 10.0f),
+                                        fminf(p.sc.env_b * thr.z, 10.0f)));
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) s_hits[warp] = __popc(mask);
+        __syncthreads();
+        uint32_t before = 0;
+        hits = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kShadeThreads / 32; w++) {
+            const uint32_t c = s_hits[w];
+            if (w < warp) before += c;
+            hits += c;
+        }
+        if (hit) s_slot[before + __popc(mask & lanemask_lt())] = uint8_t(threadIdx.x);
+        __syncthreads();
+    }
+    if (hits == 0) return;
+    if (threadIdx.x < hits) {
+        const uint32_t i = first + s_slot[threadIdx.x];
         const float4 h0 = p.hits_in[size_t(i) * 2];
         const int32_t triPtr = __float_as_int(h0.y);
         const float4 pay = p.pay_in[i];
         const uint32_t pix = __float_as_uint(pay.w);
         V3 thr = v3(pay.x, pay.y, pay.z);
-        const bool gbuffer = p.gb_write && p.bounce == 0;
-        if (gbuffer && triPtr < 0) {
-            const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
-            write_gbuffer(p, pix & kPixelMask, false, ld3(o4) + ld3(d4) * 100.0f, v3(1.0f, 0.0f, 0.0f), 0, 0);
-        }
-        if (triPtr < 0 && p.sc.env_r + p.sc.env_g + p.sc.env_b > 0.0f) {
-            // EvaluateBounce's miss: the environment times the throughput, clamped per channel
-            add_radiance(p, pix, v3(fminf(p.sc.env_r * thr.x, 10.0f), fminf(p.sc.env_g * thr.y, 10.0f),
-                                    fminf(p.sc.env_b * thr.z, 10.0f)));
-        }
-        if (triPtr >= 0) {
+        {
             const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
             const float4 h1 = p.hits_in[size_t(i) * 2 + 1];
             Surf sf = make_surface(p.sc, ld3(o4), ld3(d4), h0.x, __float_as_int(h0.z), triPtr, h1.x, h1.y);

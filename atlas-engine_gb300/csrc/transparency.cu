@@ -32,7 +32,7 @@ void* KernelFor() {
 
 ae_rt_status atlas::rt::host::TraceTransparency(ae_rt_ctx* ctx, bool any, const ae_packed_ray* rays, uint32_t n,
                                                 float tmin, float tmax, uint32_t cull_mask, void* out, void* stream,
-                                                const uint32_t* count_dev, bool per_ray_tmax) {
+                                                const uint32_t* count_dev, bool per_ray_tmax, uint32_t* counter) {
     if (!ctx) return AE_RT_INVALID_ARG;
     if (!ctx->scene_ready) return Fail(ctx, AE_RT_INVALID_ARG, "no scene has been set");
     if (n == 0) return AE_RT_OK;
@@ -81,7 +81,8 @@ ae_rt_status atlas::rt::host::TraceTransparency(ae_rt_ctx* ctx, bool any, const 
     p.hits = any ? nullptr : static_cast<float4*>(d_out);
     p.transparency = any ? static_cast<float*>(d_out) : nullptr;
     p.error_word = ctx->d_counter + 1;
-    AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
+    p.work_counter = counter;
+    if (!counter) AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
     const bool shallow = ctx->scene_depth < 32u;

@@ -137,3 +137,24 @@ def test_retest_of_any_number_of_rays_gives_the_full_records(ctx):
         ctx.retest_near_ties(mid, rays, hits, 0.0, 1e12, part, n_rays=k)
         assert torch.equal(part[:k].view(torch.int32), full[:k].view(torch.int32)), k
         assert not part[k:].any()
+
+
+@pytest.mark.parametrize("bounces", [1022, 1023, 1030])
+def test_path_tracer_counters_past_their_sets(bounces):
+    """The path tracer's per-bounce counters are used again past 1,024 bounces;
+    every path has ended long before, so the image is that of 200 bounces."""
+    import torch
+    from atlas_rt import ptscene
+    c = atlas_rt.Context(device=0)
+    try:
+        ptscene.upload(c, ptscene.build(seed=7, grid=16, n_boxes=4))
+        cam = atlas_rt.make_camera(scenes.pinhole_camera(24, 17))
+        img = []
+        for b in (200, bounces):
+            acc = torch.zeros((24 * 17, 4), device="cuda")
+            c.pathtrace(cam, acc, spp=2, max_bounces=b)
+            c.synchronize()
+            img.append(acc)
+        assert torch.equal(*img) and float(img[0].sum()) > 0
+    finally:
+        c.close()
