@@ -39,7 +39,6 @@ struct Shape {
 constexpr Shape kShapes[] = { { 4, 32 }, { 2, 32 }, { 8, 16 }, { 4, 16 } };
 constexpr int kNumShapes = 4;
 
-using atlas::rt::dev::MODE_BATCH;
 using atlas::rt::dev::MODE_MESH;
 using atlas::rt::dev::MODE_SCENE;
 
@@ -47,12 +46,11 @@ template <bool ANY, bool COUNT, int MODE, int W, int S, bool TIES = true, int ST
           int STACK = kStackEntries, bool CAMERA = false>
 void* KernelFor() {
     // 64 registers for 32 warps an SM; the scene kernels that detect near ties
-    // and the batched ones carry more per-lane state and get 72 (at 64: 1,892
-    // against 1,842 us for the 512-instance scene, 3,046 against 3,003 us for
-    // 64 meshes; the scene kernels without ties gain, a path-traced sample
-    // 1,378 against 1,410 us).  36 or 40 warps of single-mesh kernels lose to
+    // carry more per-lane state and get 72 (at 64: 1,892 against 1,842 us for
+    // the 512-instance scene; those without ties gain from 64, a path-traced
+    // sample 1,378 against 1,410 us).  36 or 40 warps of single-mesh kernels lose to
     // spills (1,126 against 1,074 us for a million random closest hits).
-    constexpr bool wide = MODE == MODE_BATCH || (MODE == MODE_SCENE && TIES && !ANY);
+    constexpr bool wide = MODE == MODE_SCENE && TIES && !ANY;
     constexpr int minBlocks = wide ? (28 / W > 0 ? 28 / W : 1) : 32 / W;
     return reinterpret_cast<void*>(
         &atlas::rt::dev::trace_kernel<ANY, COUNT, MODE, W, S, STACK - S, minBlocks, false, TIES && !ANY, STAGE, LOOSE,
@@ -81,7 +79,7 @@ void* PickShape(bool any, bool count, int mode, bool ties, bool staged, bool loo
     if (loose && mode == MODE_MESH && !count && !staged)
         return any ? KernelFor<true, false, MODE_MESH, W, S, false, 0, true, STACK>()
                    : KernelFor<false, false, MODE_MESH, W, S, false, 0, true, STACK>();
-    if (staged && !count && mode != MODE_BATCH) {
+    if (staged && !count) {
         if (mode == MODE_SCENE) {
             if (any) return KernelFor<true, false, MODE_SCENE, W, S, true, T>();
             return ties ? KernelFor<false, false, MODE_SCENE, W, S, true, T>()
@@ -90,11 +88,6 @@ void* PickShape(bool any, bool count, int mode, bool ties, bool staged, bool loo
         if (any) return KernelFor<true, false, MODE_MESH, W, S, true, T>();
         return ties ? KernelFor<false, false, MODE_MESH, W, S, true, T>()
                     : KernelFor<false, false, MODE_MESH, W, S, false, T>();
-    }
-    if (mode == MODE_BATCH) {
-        if (count) return ties ? KernelFor<false, true, MODE_BATCH, W, S>() : KernelFor<false, true, MODE_BATCH, W, S, false>();
-        return ties ? KernelFor<false, false, MODE_BATCH, W, S, true, 0, false, STACK>()
-                    : KernelFor<false, false, MODE_BATCH, W, S, false, 0, false, STACK>();
     }
     if (mode == MODE_SCENE) {
         if (count)
@@ -138,6 +131,28 @@ void* PickKernelShape(int shape, uint32_t depth, bool any, bool count, int mode,
     case 3: return PickShape<4, 16, kStackEntries>(any, count, mode, ties, staged, loose, camera);
     default: return shallow ? PickShape<4, 32, 32>(any, count, mode, ties, staged, loose, camera)
                             : PickShape<4, 32, kStackEntries>(any, count, mode, ties, staged, loose, camera);
+    }
+}
+
+// The batched launch's kernel: 72 registers.
+template <int W, int S, int STACK>
+void* PickBatchStack(bool count, bool ties) {
+    using atlas::rt::dev::batch_kernel;
+    constexpr int B = 28 / W > 0 ? 28 / W : 1;
+    if (count)
+        return ties ? reinterpret_cast<void*>(&batch_kernel<true, W, S, kStackEntries - S, B, true>)
+                    : reinterpret_cast<void*>(&batch_kernel<true, W, S, kStackEntries - S, B, false>);
+    return ties ? reinterpret_cast<void*>(&batch_kernel<false, W, S, STACK - S, B, true>)
+                : reinterpret_cast<void*>(&batch_kernel<false, W, S, STACK - S, B, false>);
+}
+
+void* PickBatch(int shape, uint32_t depth, bool count, bool ties) {
+    const bool shallow = depth < uint32_t(kShapes[shape].smem);
+    switch (shape) {
+    case 1: return shallow ? PickBatchStack<2, 32, 32>(count, ties) : PickBatchStack<2, 32, kStackEntries>(count, ties);
+    case 2: return PickBatchStack<8, 16, kStackEntries>(count, ties);
+    case 3: return PickBatchStack<4, 16, kStackEntries>(count, ties);
+    default: return shallow ? PickBatchStack<4, 32, 32>(count, ties) : PickBatchStack<4, 32, kStackEntries>(count, ties);
     }
 }
 
@@ -258,8 +273,7 @@ cudaError_t atlas::rt::host::NextWorkCounter(ae_rt_ctx* ctx, cudaStream_t s, uin
 
 namespace {
 
-// depth: stack entries the launch's trees can need (batched launches hold
-// kStackEntries at most and report overflow beyond).
+// depth: stack entries the launch's trees can need.
 // p.work_counter: a word that an earlier kernel on `s` zeroed, or null (one of
 // the context's).
 // camera: the rays are p.cam's camera rays (single mesh, closest hit, a tree
@@ -270,7 +284,7 @@ ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStre
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
-    const bool deep = depth > uint32_t(kStackEntries) && mode != MODE_BATCH;
+    const bool deep = depth > uint32_t(kStackEntries);
     void* fn = deep ? PickDeep(any, mode, ties && ctx->near_ties)
                     : PickKernelShape(ctx->shape, depth, any, ctx->count_fetches, mode, ties && ctx->near_ties,
                                       ctx->staged_rays, ctx->approximate, camera);
@@ -748,62 +762,83 @@ ae_rt_status ae_rt_trace_scene_any_queue(ae_rt_ctx* ctx, const ae_packed_ray* ra
 
 struct ae_rt_batch_plan {
     ae_rt_ctx* ctx = nullptr;
-    atlas::rt::dev::BatchDesc* d_batches = nullptr;
-    uint32_t* d_counter = nullptr;
-    uint32_t n_batches = 0;
-    uint32_t total = 0;
+    atlas::rt::dev::BatchDesc* d_batches = nullptr;     // the table, then two work counters
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
 
 namespace {
 
-// Device batch table for a launch, its total ray count and the depth of its
-// deepest tree.
-ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32_t n,
-                            std::vector<atlas::rt::dev::BatchDesc>& table, uint32_t& total, uint32_t& depth) {
-    depth = 0;
-    table.resize(n);
-    uint64_t first = 0;
+// Device batch table of a launch: the closest-hit batches, then the any-hit
+// ones, each kind with its own global ray numbering.
+struct BatchTable {
+    std::vector<atlas::rt::dev::BatchDesc> desc;
+    uint32_t n_closest = 0;            // descriptors of closest-hit batches
+    uint32_t rays[2] = { 0, 0 };       // closest, any
+    uint32_t depth = 0;                // of the deepest tree
+};
+
+ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32_t n, BatchTable& t) {
+    uint64_t total = 0;
     for (uint32_t i = 0; i < n; i++) {
         const ae_batch_desc& b = batches[i];
         if (b.mesh_id < 0 || size_t(b.mesh_id) >= ctx->meshes.size())
             return Fail(ctx, AE_RT_INVALID_ARG, "batch " + std::to_string(i) + ": unknown mesh id");
         if (b.n_rays && (!IsDevicePointer(b.rays) || !IsDevicePointer(b.out)))
             return Fail(ctx, AE_RT_INVALID_ARG, "batch " + std::to_string(i) + ": batched traces take device buffers");
-        const DeviceMesh& m = ctx->meshes[size_t(b.mesh_id)];
-        atlas::rt::dev::BatchDesc& d = table[i];
-        depth = std::max(depth, m.depth);
-        d.nodes = m.nodes;
-        d.tris = m.tris;
-        d.rays = reinterpret_cast<const float4*>(b.rays);
-        d.out = b.out;
-        d.n_nodes = m.n_nodes;
-        d.n_tris = m.n_tris;
-        d.n_rays = b.n_rays;
-        d.any = b.any ? 1u : 0u;
-        d.tmin = b.tmin;
-        d.tmax = b.tmax;
-        d.first = uint32_t(first);
-        d.max_steps = ctx->max_steps_cfg ? ctx->max_steps_cfg : MaxSteps(ctx, m);
-        first += b.n_rays;
-        if (first > (1u << 30)) return Fail(ctx, AE_RT_INVALID_ARG, "more than 2^30 rays in one batched launch");
+        total += b.n_rays;
+        if (total > (1u << 30)) return Fail(ctx, AE_RT_INVALID_ARG, "more than 2^30 rays in one batched launch");
     }
-    total = uint32_t(first);
+    t.desc.reserve(n);
+    for (int any = 0; any < 2; any++) {
+        if (any) t.n_closest = uint32_t(t.desc.size());
+        for (uint32_t i = 0; i < n; i++) {
+            const ae_batch_desc& b = batches[i];
+            if ((b.any != 0) != (any != 0)) continue;
+            const DeviceMesh& m = ctx->meshes[size_t(b.mesh_id)];
+            atlas::rt::dev::BatchDesc d{};
+            d.nodes = m.nodes;
+            d.tris = m.tris;
+            d.rays = reinterpret_cast<const float4*>(b.rays);
+            d.out = b.out;
+            d.n_nodes = m.n_nodes;
+            d.n_tris = m.n_tris;
+            d.n_rays = b.n_rays;
+            d.any = uint32_t(any);
+            d.tmin = b.tmin;
+            d.tmax = b.tmax;
+            d.first = t.rays[any];
+            d.max_steps = MaxSteps(ctx, m);
+            t.rays[any] += b.n_rays;
+            t.depth = std::max(t.depth, m.depth);
+            t.desc.push_back(d);
+        }
+    }
     return AE_RT_OK;
 }
 
-TraceParams BatchParams(ae_rt_ctx* ctx, const atlas::rt::dev::BatchDesc* d_batches, uint32_t n, uint32_t total) {
-    TraceParams p{};
-    p.n_rays = total;
-    p.error_word = ctx->d_counter + 1;
-    p.fetch_counts = ctx->d_fetch;
-    p.batches = d_batches;
-    p.n_batches = n;
-    p.refill_steps = ctx->refill_steps;
-    p.spread_warps = SpreadWarps(ctx);
-    p.max_steps = 0xffffffffu;
-    return p;
+// The batched launch over a device copy of `t.desc`; counters: two words;
+// count: fetch totals.
+cudaError_t LaunchBatches(ae_rt_ctx* ctx, const BatchTable& t, const atlas::rt::dev::BatchDesc* d_desc,
+                          uint32_t* counters, bool count, cudaStream_t s) {
+    TraceParams p[2] = {};
+    for (int any = 0; any < 2; any++) {
+        p[any].n_rays = t.rays[any];
+        p[any].work_counter = counters + any;
+        p[any].error_word = ctx->d_counter + 1;
+        p[any].fetch_counts = ctx->d_fetch;
+        p[any].batches = d_desc + (any ? t.n_closest : 0u);
+        p[any].n_batches = any ? uint32_t(t.desc.size()) - t.n_closest : t.n_closest;
+        p[any].refill_steps = ctx->refill_steps;
+        p[any].spread_warps = SpreadWarps(ctx);
+        p[any].max_steps = 0xffffffffu;
+    }
+    cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    void* fn = PickBatch(ctx->shape, t.depth, count, ctx->near_ties);
+    void* args[] = { &p[0], &p[1] };
+    const size_t stacks = size_t(ctx->threads) * size_t(kShapes[ctx->shape].smem) * sizeof(int32_t);
+    return cudaLaunchKernel(fn, dim3(GridFor(ctx, fn, t.rays[0] + t.rays[1])), dim3(ctx->threads), args, stacks, s);
 }
 
 }  // namespace
@@ -813,18 +848,20 @@ ae_rt_status ae_rt_trace_batched(ae_rt_ctx* ctx, const ae_batch_desc* batches, u
     if (n_batches == 0) return AE_RT_OK;
     if (!batches) return Fail(ctx, AE_RT_INVALID_ARG, "null batch table");
     AE_CUDA(ctx, cudaSetDevice(ctx->device));
-    std::vector<atlas::rt::dev::BatchDesc> table;
-    uint32_t total = 0, depth = 0;
-    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total, depth);
+    BatchTable t;
+    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, t);
     if (st != AE_RT_OK) return st;
-    if (total == 0) return AE_RT_OK;
+    if (t.rays[0] + t.rays[1] == 0) return AE_RT_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    AE_CUDA(ctx, ctx->batch_table.ensure(table.size() * sizeof(table[0])));
-    AE_CUDA(ctx, cudaMemcpyAsync(ctx->batch_table.ptr, table.data(), table.size() * sizeof(table[0]),
-                                 cudaMemcpyHostToDevice, s));
-    TraceParams p = BatchParams(ctx, static_cast<atlas::rt::dev::BatchDesc*>(ctx->batch_table.ptr), n_batches,
-                                total);
-    return Launch(ctx, false, MODE_BATCH, p, s, true, depth);
+    // the table, then the two work counters
+    const size_t bytes = t.desc.size() * sizeof(t.desc[0]);
+    AE_CUDA(ctx, ctx->batch_table.ensure(bytes + 2 * sizeof(uint32_t)));
+    auto* d_desc = static_cast<atlas::rt::dev::BatchDesc*>(ctx->batch_table.ptr);
+    AE_CUDA(ctx, cudaMemcpyAsync(d_desc, t.desc.data(), bytes, cudaMemcpyHostToDevice, s));
+    if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
+    AE_CUDA(ctx, LaunchBatches(ctx, t, d_desc, reinterpret_cast<uint32_t*>(d_desc + t.desc.size()),
+                               ctx->count_fetches, s));
+    return AE_RT_OK;
 }
 
 ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32_t n_batches,
@@ -833,30 +870,22 @@ ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batche
     *out = nullptr;
     if (n_batches == 0 || !batches) return Fail(ctx, AE_RT_INVALID_ARG, "a plan needs at least one batch");
     AE_CUDA(ctx, cudaSetDevice(ctx->device));
-    std::vector<atlas::rt::dev::BatchDesc> table;
-    uint32_t total = 0, depth = 0;
-    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, table, total, depth);
+    BatchTable t;
+    ae_rt_status st = MakeBatchTable(ctx, batches, n_batches, t);
     if (st != AE_RT_OK) return st;
     auto* plan = new (std::nothrow) ae_rt_batch_plan;
     if (!plan) return AE_RT_OUT_OF_MEMORY;
     plan->ctx = ctx;
-    plan->n_batches = n_batches;
-    plan->total = total;
     cudaStream_t cap = nullptr;
-    cudaError_t e = cudaMalloc(&plan->d_batches, table.size() * sizeof(table[0]));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(plan->d_batches, table.data(), table.size() * sizeof(table[0]), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_counter, sizeof(uint32_t));
+    const size_t bytes = t.desc.size() * sizeof(t.desc[0]);
+    cudaError_t e = cudaMalloc(&plan->d_batches, bytes + 2 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemcpy(plan->d_batches, t.desc.data(), bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        TraceParams p = BatchParams(ctx, plan->d_batches, n_batches, total);
-        p.work_counter = plan->d_counter;
-        void* args[] = { &p };
-        void* fn = PickKernelShape(ctx->shape, depth, false, false, MODE_BATCH, ctx->near_ties);
-        cudaError_t le = cudaMemsetAsync(plan->d_counter, 0, sizeof(uint32_t), cap);
-        if (le == cudaSuccess)
-            le = cudaLaunchKernel(fn, dim3(GridFor(ctx, fn, total)), dim3(ctx->threads), args, 0, cap);
+        const cudaError_t le = LaunchBatches(ctx, t, plan->d_batches,
+                                             reinterpret_cast<uint32_t*>(plan->d_batches + t.desc.size()), false,
+                                             cap);
         e = cudaStreamEndCapture(cap, &plan->graph);
         if (le != cudaSuccess) e = le;
     }
@@ -884,7 +913,6 @@ void ae_rt_batch_plan_destroy(ae_rt_batch_plan* plan) {
     if (plan->exec) cudaGraphExecDestroy(plan->exec);
     if (plan->graph) cudaGraphDestroy(plan->graph);
     cudaFree(plan->d_batches);
-    cudaFree(plan->d_counter);
     delete plan;
 }
 

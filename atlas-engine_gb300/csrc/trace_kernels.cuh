@@ -74,7 +74,8 @@ struct TraceParams {
     const MeshDesc* meshes;      // indexed by GPUBVHInstance::meshOffset
     uint32_t n_meshes;
     uint32_t cull_mask;
-    // batched multi-mesh launches (MODE_BATCH): n_rays = total over batches
+    // batched multi-mesh launches (MODE_BATCH): n_rays = total over the batches
+    // of the query kind
     const struct BatchDesc* batches;
     uint32_t n_batches;
     uint32_t refill_steps;       // traversal steps between warp refills
@@ -681,8 +682,8 @@ static __device__ __noinline__ float texture_opacity(const float* materials, uin
 // totals.  MODE_SCENE: two-level traversal over instances (CheckInstance,
 // bvh.hsh:172-189, with the TLAS/BLAS switch keyed on the stack depth at which
 // the instance was entered, bvh.hsh:212-223).  MODE_BATCH: every lane finds
-// its ray's batch (mesh, query kind, t range, result buffer) when it takes a
-// ray, so one launch serves many meshes and both query kinds.
+// its ray's batch (mesh, t range, result buffer) when it takes a ray, so one
+// launch serves many meshes.
 // BOUNDS = true adds range checks of every node and triangle index against
 // n_nodes / n_tris (for callers whose BVH did not pass the host validator);
 // an out-of-range index ends the ray with the overflow flag set.
@@ -714,29 +715,31 @@ static __device__ __noinline__ float texture_opacity(const float* materials, uin
 // CAMERA: ray i is the camera ray of queue slot i (camera_ray), made by the
 // lane that takes it, instead of a load from a ray buffer written by a
 // separate ray-generation launch.
-template <bool ANY, bool COUNT, int MODE, int WARPS, int SMEM_STACK, int SPILL_STACK, int MIN_BLOCKS,
-          bool BOUNDS = false, bool TIES = true, int STAGE = 0, bool LOOSE = false, bool CAMERA = false,
-          bool OPACITY = false>
-__global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TraceParams p) {
+template <bool ANY, bool COUNT, int MODE, int WARPS, int SMEM_STACK, int SPILL_STACK, bool BOUNDS, bool TIES,
+          int STAGE, bool LOOSE, bool CAMERA, bool OPACITY>
+__device__ __forceinline__ void trace_rays(const TraceParams& p) {
     constexpr bool TLAS = MODE == MODE_SCENE;
     constexpr bool BATCH = MODE == MODE_BATCH;
     static_assert(STAGE == 0 || (!BATCH && !BOUNDS), "staged rays: single-mesh and scene launches only");
     static_assert(!LOOSE || (!TIES && !BOUNDS), "loose traversal: no near-tie flag, uploaded nodes");
     static_assert(!OPACITY || (TLAS && !TIES && !LOOSE && !COUNT && !BOUNDS && STAGE == 0), "transparency: exact scenes");
     static_assert(!CAMERA || (MODE == MODE_MESH && STAGE == 0 && !ANY), "camera rays: single-mesh closest hits");
-    __shared__ int32_t s_stack[WARPS][SMEM_STACK][32];
+    // the batched launch's two loops share their stacks: dynamic shared memory
+    __shared__ int32_t s_stack[BATCH ? 1 : WARPS][BATCH ? 1 : SMEM_STACK][32];
+    extern __shared__ int32_t s_batch_stack[];
     // scenes: the world-space ray of each lane while it is inside an instance
     // (held in registers beside the object-space one it cost spills, and every
     // step selected between the two)
     __shared__ uint32_t s_world[TLAS ? WARPS : 1][TLAS ? 10 : 1][32];
     __shared__ __align__(128) float4 s_rays[STAGE > 0 ? WARPS : 1][2][STAGE > 0 ? STAGE * 3 : 1];
     __shared__ __align__(8) uint64_t s_rbar[STAGE > 0 ? WARPS : 1][2];
+    __shared__ uint32_t s_rstate[STAGE > 0 ? WARPS : 1][3];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = threadIdx.x >> 5;
     constexpr unsigned kFull = 0xffffffffu;
 
     LaneStack<SMEM_STACK, SPILL_STACK> st;
-    st.sh = &s_stack[warp][0][lane];
+    st.sh = BATCH ? s_batch_stack + warp * (SMEM_STACK * 32) + lane : &s_stack[BATCH ? 0 : warp][0][lane];
     st.put(0, kStackEnd);
 
     bool live = false;
@@ -751,7 +754,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     const float4* blasTris = p.tris;
     bool occl = false;
     bool tieSuspect = false;        // closest hit: a near tie the second distance cannot show (kTieWindow)
-    bool laneAny = ANY;             // batched: the lane's query kind
     float tmin = p.tmin, tmax = p.tmax;
     uint32_t maxSteps = p.max_steps;
     void* out = nullptr;            // batched: the lane's result array
@@ -818,7 +820,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
     // tile sits in buffer kStCur's value, the next in the other one
     constexpr uint32_t kStUsed = 0xffu, kStCur = 1u << 8, kStPhase0 = 1u << 9, kStPending = 1u << 11,
                        kStDry = 1u << 12, kStFault = 1u << 13, kStEmpty = 1u << 14;
-    __shared__ uint32_t s_rstate[STAGE > 0 ? WARPS : 1][3];
     if constexpr (STAGE > 0) {
         if (lane == 0) {
             stage_barrier_init(shared_addr(&s_rbar[warp][0]));
@@ -917,7 +918,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                             nodes = bd.nodes;
                             blasTris = bd.tris;
                             nodesHere = bd.n_nodes;
-                            laneAny = bd.any != 0;
                             tmin = bd.tmin;
                             tmax = bd.tmax;
                             maxSteps = bd.max_steps;
@@ -942,7 +942,6 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
 
         // ---- traverse: a bounded number of steps, then refill again ----
         if (live) {
-            const bool anyQ = ANY || (BATCH && laneAny);
             // the burst ends after `burst` steps or at the ray's step cap
             const uint32_t lim = min(steps + burst, maxSteps);
             while (node != kStackEnd) {
@@ -1021,7 +1020,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                                     hitDist = t; hitID = tp; hu = u; hv = v; hitInst = curInst;
                                 }
                             }
-                        } else if (anyQ) {
+                        } else if (ANY) {
                             if (hit && t > tmin && t < tmax) { occl = true; end = true; }
                         } else if (hit && t > tmin && t < tmax) {
                             if (t < hitDist) {
@@ -1040,7 +1039,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                         if (transparency < 0.000001f) transparency = 0.0f;
                         occl = !(transparency > 0.0f);
                     }
-                    if ((BOUNDS && (flags & kHitFlagOverflow)) || (anyQ && occl)) node = kStackEnd;
+                    if ((BOUNDS && (flags & kHitFlagOverflow)) || (ANY && occl)) node = kStackEnd;
                     else node = st.get(--sp);
                 } else {
                     const float4* np = nodes + size_t(node) * 4;
@@ -1049,16 +1048,12 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
                     const int32_t lptr = n.lptr, rptr = n.rptr;
                     bool il, ir, leftFirst, nearCull = false;
                     if (LOOSE)
-                        test_children_loose(r, n, tmin, anyQ ? tmax : hitDist, il, ir, leftFirst);
+                        test_children_loose(r, n, tmin, ANY ? tmax : hitDist, il, ir, leftFirst);
                     else
-                        // the batched launch decides the query kind per lane at run time; with
-                        // both box tests compiled into it, it ran 8 % slower (11.85 against
-                        // 10.99 ms on 64 meshes), so every lane takes the exact test there
-                        test_children(r, n, tmin, anyQ ? tmax : hitDist, BATCH || !anyQ, TIES && !anyQ, il, ir,
-                                      leftFirst, nearCull);
-                    if (TIES && !anyQ) tieSuspect = tieSuspect || nearCull;
+                        test_children(r, n, tmin, ANY ? tmax : hitDist, !ANY, TIES && !ANY, il, ir, leftFirst, nearCull);
+                    if (TIES && !ANY) tieSuspect = tieSuspect || nearCull;
                     int32_t next, far;
-                    if (anyQ) {
+                    if (ANY) {
                         next = il ? lptr : rptr;
                         far = rptr;
                     } else {
@@ -1093,7 +1088,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
             if (node == kStackEnd) {
                 if (OPACITY && ANY) {
                     p.transparency[rid] = transparency;
-                } else if (anyQ) {
+                } else if (ANY) {
                     uint8_t* occOut = BATCH ? static_cast<uint8_t*>(out) : p.occluded;
                     occOut[rid] = (occl && !(flags & (kHitFlagOverflow | kHitFlagIterCap))) ? 1 : 0;
                 } else {
@@ -1132,6 +1127,25 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TracePara
             atomicAdd(p.fetch_counts + 1, tc);
         }
     }
+}
+
+template <bool ANY, bool COUNT, int MODE, int WARPS, int SMEM_STACK, int SPILL_STACK, int MIN_BLOCKS,
+          bool BOUNDS = false, bool TIES = true, int STAGE = 0, bool LOOSE = false, bool CAMERA = false,
+          bool OPACITY = false>
+__global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TraceParams p) {
+    trace_rays<ANY, COUNT, MODE, WARPS, SMEM_STACK, SPILL_STACK, BOUNDS, TIES, STAGE, LOOSE, CAMERA, OPACITY>(p);
+}
+
+// One launch over batches of both query kinds: every warp takes closest-hit
+// rays until none is left, then any-hit rays, so that either loop is compiled
+// for its kind alone (the any-hit one with the screened box test; with the
+// kind decided per lane, 64 meshes took 3,020 instead of 2,801 us).
+template <bool COUNT, int WARPS, int SMEM_STACK, int SPILL_STACK, int MIN_BLOCKS, bool TIES>
+__global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) batch_kernel(TraceParams closest, TraceParams any) {
+    if (closest.n_rays)
+        trace_rays<false, COUNT, MODE_BATCH, WARPS, SMEM_STACK, SPILL_STACK, false, TIES, 0, false, false, false>(closest);
+    if (any.n_rays)
+        trace_rays<true, COUNT, MODE_BATCH, WARPS, SMEM_STACK, SPILL_STACK, false, false, 0, false, false, false>(any);
 }
 
 }  // namespace atlas::rt::dev

@@ -158,3 +158,32 @@ def test_path_tracer_counters_past_their_sets(bounces):
         assert torch.equal(*img) and float(img[0].sum()) > 0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("kinds", ["c", "a", "ac", "ca", "acca0c", "0a", "c0"])
+def test_batches_of_either_kind_alone_and_mixed(few, kinds):
+    """Batched launches (direct and planned) with closest-hit (c), any-hit (a)
+    and empty (0) batches in any order: each gives its single launch's records."""
+    torch = few["torch"]
+    c, rays = few["ctx"], few["rays"]
+    batches, want = [], []
+    for i, k in enumerate(kinds):
+        n = 0 if k == "0" else 700 * i + 33
+        at = 5000 * i
+        any_hit = k == "a" or (k == "0" and i % 2 == 1)
+        out = torch.full((max(n, 1),), 7, dtype=torch.uint8, device="cuda") if any_hit \
+            else torch.zeros((max(n, 1), 8), device="cuda")
+        batches.append({"mesh": few["mid"], "any": any_hit, "rays": rays[at:], "out": out, "n_rays": n, "tmin": 1e-4,
+                        "tmax": 10.0})
+        want.append(few["full"]["any" if any_hit else "closest"][at:at + n])
+    plan = c.batch_plan(batches)
+    for launch in (lambda: c.trace_batched(batches), plan.launch, plan.launch):
+        for b in batches:
+            b["out"].zero_()
+        launch()
+        c.synchronize()
+        for b, w in zip(batches, want):
+            got = b["out"][:b["n_rays"]]
+            got = got if b["any"] else got.view(torch.int32)
+            assert np.array_equal(got.cpu().numpy().reshape(w.shape), w)
+    plan.close()
