@@ -43,7 +43,7 @@ using atlas::rt::dev::MODE_MESH;
 using atlas::rt::dev::MODE_SCENE;
 
 template <bool ANY, bool COUNT, int MODE, int W, int S, bool TIES = true, int STAGE = 0, bool LOOSE = false,
-          int STACK = kStackEntries, bool CAMERA = false>
+          int STACK = kStackEntries, bool CAMERA = false, bool FEW = false>
 void* KernelFor() {
     // 64 registers for 32 warps an SM; the scene kernels that detect near ties
     // carry more per-lane state and get 72 (at 64: 1,892 against 1,842 us for
@@ -54,7 +54,7 @@ void* KernelFor() {
     constexpr int minBlocks = wide ? (28 / W > 0 ? 28 / W : 1) : 32 / W;
     return reinterpret_cast<void*>(
         &atlas::rt::dev::trace_kernel<ANY, COUNT, MODE, W, S, STACK - S, minBlocks, false, TIES && !ANY, STAGE, LOOSE,
-                                      CAMERA>);
+                                      CAMERA, false, FEW>);
 }
 
 // ties = false: the caller discards the near-tie flag (the library's path
@@ -117,6 +117,20 @@ void* PickDeep(bool any, int mode, bool ties) {
     if (any) return KernelFor<true, false, MODE_MESH, 4, 32, true, 0, false, kDeepStackEntries>();
     return ties ? KernelFor<false, false, MODE_MESH, 4, 32, true, 0, false, kDeepStackEntries>()
                 : KernelFor<false, false, MODE_MESH, 4, 32, false, 0, false, kDeepStackEntries>();
+}
+
+// Launches of few rays, default shape, trees of fewer than 32 levels, exact,
+// no counters; null for any other launch.
+void* PickFew(int shape, uint32_t depth, bool any, int mode, bool ties) {
+    if (shape != 0 || depth >= uint32_t(kShapes[0].smem)) return nullptr;
+    if (mode == MODE_SCENE) {
+        if (any) return KernelFor<true, false, MODE_SCENE, 4, 32, true, 0, false, 32, false, true>();
+        return ties ? KernelFor<false, false, MODE_SCENE, 4, 32, true, 0, false, 32, false, true>()
+                    : KernelFor<false, false, MODE_SCENE, 4, 32, false, 0, false, 32, false, true>();
+    }
+    if (any) return KernelFor<true, false, MODE_MESH, 4, 32, true, 0, false, 32, false, true>();
+    return ties ? KernelFor<false, false, MODE_MESH, 4, 32, true, 0, false, 32, false, true>()
+                : KernelFor<false, false, MODE_MESH, 4, 32, false, 0, false, 32, false, true>();
 }
 
 // depth: the stack entries that the launch's trees can need (at most
@@ -280,7 +294,6 @@ namespace {
 // within kStackEntries, exact, no counters: Trace checks this).
 ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStream_t s, bool ties, uint32_t depth,
                     bool camera = false) {
-    if (!p.work_counter) AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
@@ -289,7 +302,22 @@ ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStre
                     : PickKernelShape(ctx->shape, depth, any, ctx->count_fetches, mode, ties && ctx->near_ties,
                                       ctx->staged_rays, ctx->approximate, camera);
     const uint32_t threads = deep ? 128u : ctx->threads;
-    const uint32_t grid = GridFor(ctx, fn, p.n_rays, threads);
+    uint32_t grid = GridFor(ctx, fn, p.n_rays, threads);
+    bool few_rays = false;
+    if (!p.n_rays_dev && !p.work_counter && !camera && !ctx->count_fetches && !ctx->staged_rays && !ctx->approximate &&
+        p.n_rays <= p.spread_warps * 32u) {
+        if (void* few = PickFew(ctx->shape, depth, any, mode, ties && ctx->near_ties)) {
+            // the warps of this grid must hold every ray (a configured blocks_per_sm can make it smaller)
+            const uint32_t few_grid = GridFor(ctx, few, p.n_rays);
+            if (uint64_t(p.n_rays) <= uint64_t(few_grid) * threads) {
+                fn = few;
+                grid = few_grid;
+                few_rays = true;
+            }
+        }
+    }
+    if (!p.work_counter && !few_rays)
+        AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     void* args[] = { &p };
     AE_CUDA(ctx, cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, 0, s));
     return AE_RT_OK;

@@ -187,3 +187,16 @@ def test_batches_of_either_kind_alone_and_mixed(few, kinds):
             got = got if b["any"] else got.view(torch.int32)
             assert np.array_equal(got.cpu().numpy().reshape(w.shape), w)
     plan.close()
+
+
+@pytest.mark.parametrize("n", [1, 19455, 19456, 19457, 38912])
+def test_few_rays_on_a_context_of_one_cta_per_sm(few, n):
+    """With one CTA an SM configured, the grid of a small launch may not hold all
+    of its rays at once (152 x 128): both sides of that line."""
+    c = atlas_rt.Context(device=0, blocks_per_sm=1)
+    try:
+        mid = c.upload_mesh(few["bvh"].nodes, few["gt"])
+        assert np.array_equal(run({**few, "ctx": c, "mid": mid}, "closest", n)[:n], few["full"]["closest"][:n])
+        assert np.array_equal(run({**few, "ctx": c, "mid": mid}, "any", n)[:n], few["full"]["any"][:n])
+    finally:
+        c.close()
