@@ -1232,7 +1232,8 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
     }
     // every queue holds at most one ray per pixel of the tile
     const uint32_t blocks = (n_tile + 255) / 256;
-    const uint32_t shade_blocks = (n_tile + atlas::rt::dev::kShadeThreads - 1) / atlas::rt::dev::kShadeThreads;
+    const uint32_t shade_blocks = std::min((n_tile + atlas::rt::dev::kShadeThreads - 1) / atlas::rt::dev::kShadeThreads,
+                                           uint32_t(ctx->sm_count) * atlas::rt::dev::kShadeCtas);
     // counters of one sample, set by its ray generation: per bounce the queue's
     // length, its shadow queue's and the work counters of the two traces (a
     // memset for each was a stream operation of its own)

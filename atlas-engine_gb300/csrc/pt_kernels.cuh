@@ -790,116 +790,123 @@ __device__ __forceinline__ void write_gbuffer(const PtParams& p, uint32_t pix, b
     }
 }
 
-// Threads of pt_shade_kernel's blocks; 6 blocks an SM, 80 registers (256
-// threads without a register bound, 16 warps an SM: 1,336 against 1,303 us for
-// a sample at 1920 x 1080).
+// Blocks of pt_shade_kernel and how many of them an SM holds (96 registers).
+// A sample at 1920 x 1080 with 4, 5 and 6 of them: 1,310, 1,272 and 1,275 us.
 constexpr uint32_t kShadeThreads = 128;
+constexpr uint32_t kShadeCtas = 5;
 
-// The block's hits are packed to its front before they are shaded: after the
-// first bounce about half of the rays miss, here and there, and a warp shaded
-// 10 of 32 lanes (22 packed: the second bounce's shading 126 -> 116 us, the
-// third's 46 -> 39, the fourth's 25 -> 18).
-static __global__ void __launch_bounds__(kShadeThreads, 6) pt_shade_kernel(PtParams p) {
-    __shared__ uint32_t s_hits[kShadeThreads / 32 + 1];
-    __shared__ uint8_t s_slot[kShadeThreads];
+// A block collects hits from chunks of its queue until every thread has one,
+// and shades them; misses are resolved as their chunk is read.  After the
+// first bounce about half of the rays miss, here and there: a warp shaded 10
+// of 32 lanes, and with each block's 128 rays packed to its front two of its
+// four warps idled at the append's barrier (the second bounce's shading 126 us
+// without packing, 97 packed; the whole sample 1,307 -> 1,272 us with the
+// chunks of a persistent grid).  Bound by instruction issue and by the latency
+// of the triangle's and the material's dependent loads.
+static __global__ void __launch_bounds__(kShadeThreads, kShadeCtas) pt_shade_kernel(PtParams p) {
+    __shared__ uint32_t s_hits[kShadeThreads / 32];
+    __shared__ uint32_t s_item[2 * kShadeThreads];   // hits waiting to be shaded
     const uint32_t n = min(*p.n_in, queue_capacity(p));
-    const uint32_t first = blockIdx.x * kShadeThreads;
-    if (first >= n) return;
-    bool emitRay = false, emitShadow = false;
-    float4 outRay0{}, outRay1{}, outPay{}, shRay0{}, shRay1{}, shPay{};
     const bool gbuffer = p.gb_write && p.bounce == 0;
-    uint32_t hits;
-    {
-        const uint32_t i = first + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-        const bool hit = i < n && __float_as_int(p.hits_in[size_t(i) * 2].y) >= 0;
-        if (i < n && !hit) {
+    uint32_t waiting = 0;
+    uint32_t first = blockIdx.x * kShadeThreads;
+    while (true) {
+        while (waiting < kShadeThreads && first < n) {
+            const uint32_t i = first + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+            const bool hit = i < n && __float_as_int(p.hits_in[size_t(i) * 2].y) >= 0;
+            if (i < n && !hit) {
+                const float4 pay = p.pay_in[i];
+                const uint32_t pix = __float_as_uint(pay.w);
+                const V3 thr = v3(pay.x, pay.y, pay.z);
+                if (gbuffer) {
+                    const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
+                    write_gbuffer(p, pix & kPixelMask, false, ld3(o4) + ld3(d4) * 100.0f, v3(1.0f, 0.0f, 0.0f), 0, 0);
+                }
+                // EvaluateBounce's miss: the environment times the throughput, clamped per channel
+                if (p.sc.env_r + p.sc.env_g + p.sc.env_b > 0.0f)
+                    add_radiance(p, pix, v3(fminf(p.sc.env_r * thr.x, 10.0f), fminf(p.sc.env_g * thr.y, 10.0f),
+                                            fminf(p.sc.env_b * thr.z, 10.0f)));
+            }
+            const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+            if (lane == 0) s_hits[warp] = __popc(mask);
+            __syncthreads();
+            uint32_t before = waiting;
+#pragma unroll
+            for (uint32_t w = 0; w < kShadeThreads / 32; w++) {
+                const uint32_t c = s_hits[w];
+                if (w < warp) before += c;
+                waiting += c;
+            }
+            if (hit) s_item[before + __popc(mask & lanemask_lt())] = i;
+            __syncthreads();
+            first += gridDim.x * kShadeThreads;
+        }
+        if (waiting == 0) return;
+        const uint32_t take = min(waiting, kShadeThreads);
+        waiting -= take;
+        bool emitRay = false, emitShadow = false;
+        float4 outRay0{}, outRay1{}, outPay{}, shRay0{}, shRay1{}, shPay{};
+        if (threadIdx.x < take) {
+            const uint32_t i = s_item[waiting + threadIdx.x];
+            const float4 h0 = p.hits_in[size_t(i) * 2];
+            const int32_t triPtr = __float_as_int(h0.y);
             const float4 pay = p.pay_in[i];
             const uint32_t pix = __float_as_uint(pay.w);
-            const V3 thr = v3(pay.x, pay.y, pay.z);
-            if (gbuffer) {
+            V3 thr = v3(pay.x, pay.y, pay.z);
+            {
                 const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
-                write_gbuffer(p, pix & kPixelMask, false, ld3(o4) + ld3(d4) * 100.0f, v3(1.0f, 0.0f, 0.0f), 0, 0);
-            }
-            // EvaluateBounce's miss: the environment times the throughput, clamped per channel
-            if (p.sc.env_r + p.sc.env_g + p.sc.env_b > 0.0f)
-                add_radiance(p, pix, v3(fminf(p.sc.env_r * thr.x, 10.0f), fminf(p.sc.env_g * thr.y, 10.0f),
-                                        fminf(p.sc.env_b * thr.z, 10.0f)));
-        }
-        const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) s_hits[warp] = __popc(mask);
-        __syncthreads();
-        uint32_t before = 0;
-        hits = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < kShadeThreads / 32; w++) {
-            const uint32_t c = s_hits[w];
-            if (w < warp) before += c;
-            hits += c;
-        }
-        if (hit) s_slot[before + __popc(mask & lanemask_lt())] = uint8_t(threadIdx.x);
-        __syncthreads();
-    }
-    if (hits == 0) return;
-    if (threadIdx.x < hits) {
-        const uint32_t i = first + s_slot[threadIdx.x];
-        const float4 h0 = p.hits_in[size_t(i) * 2];
-        const int32_t triPtr = __float_as_int(h0.y);
-        const float4 pay = p.pay_in[i];
-        const uint32_t pix = __float_as_uint(pay.w);
-        V3 thr = v3(pay.x, pay.y, pay.z);
-        {
-            const float4 o4 = p.rays_in[size_t(i) * 3], d4 = p.rays_in[size_t(i) * 3 + 1];
-            const float4 h1 = p.hits_in[size_t(i) * 2 + 1];
-            Surf sf = make_surface(p.sc, ld3(o4), ld3(d4), h0.x, __float_as_int(h0.z), triPtr, h1.x, h1.y);
-            if (gbuffer) write_gbuffer(p, pix & kPixelMask, true, sf.P, sf.geoN, sf.mat.id, __float_as_int(h0.z));
-            // emission of the first hit (rayHit.csh:180-183); with MIS, also
-            // the emission a continuation finds, weighted by its factor (ray dir.w)
-            const bool emissive = sf.mat.emissive.x + sf.mat.emissive.y + sf.mat.emissive.z > 0.0f;
-            if (p.bounce == 0 && emissive) add_radiance(p, pix, sf.mat.emissive);
-            if (p.bounce > 0 && emissive && d4.w > 0.0f) add_radiance(p, pix, thr * sf.mat.emissive * d4.w);
-            const bool cont = p.bounce < p.max_bounces;
-            V3 c, so, sd;
-            float st, pl = 0.0f;
-            if (direct_light(p.sc, sf, thr, pix, p.sample, p.bounce, p.seed, p.epsilon, c, so, sd, st, &pl)) {
-                if (p.mis && cont) c = c * power_weight(pl, bsdf_pdf(sf, sf.L));
-                emitShadow = true;
-                shRay0 = make_float4(so.x, so.y, so.z, __uint_as_float(pix));
-                shRay1 = make_float4(sd.x, sd.y, sd.z, st);
-                shPay = make_float4(c.x, c.y, c.z, __uint_as_float(pix));
-            }
-            if (cont) {
-                V3 o, d;
-                bool spec = false, passed = false;
-                if (continue_path(sf, thr, pix, p.sample, p.bounce, p.seed, p.epsilon, o, d, &spec, &passed)) {
-                    emitRay = true;
-                    outRay0 = make_float4(o.x, o.y, o.z, __uint_as_float(pix));
-                    // a light seen through a pass-through is not part of the
-                    // engine's direct light (its NEE evaluates reflection only)
-                    outRay1 = make_float4(d.x, d.y, d.z,
-                                          p.mis && !passed ? mis_hit_factor(p.sc, sf, d, spec) : 0.0f);
-                    outPay = make_float4(thr.x, thr.y, thr.z, __uint_as_float(pix));
+                const float4 h1 = p.hits_in[size_t(i) * 2 + 1];
+                Surf sf = make_surface(p.sc, ld3(o4), ld3(d4), h0.x, __float_as_int(h0.z), triPtr, h1.x, h1.y);
+                if (gbuffer) write_gbuffer(p, pix & kPixelMask, true, sf.P, sf.geoN, sf.mat.id, __float_as_int(h0.z));
+                // emission of the first hit (rayHit.csh:180-183); with MIS, also
+                // the emission a continuation finds, weighted by its factor (ray dir.w)
+                const bool emissive = sf.mat.emissive.x + sf.mat.emissive.y + sf.mat.emissive.z > 0.0f;
+                if (p.bounce == 0 && emissive) add_radiance(p, pix, sf.mat.emissive);
+                if (p.bounce > 0 && emissive && d4.w > 0.0f) add_radiance(p, pix, thr * sf.mat.emissive * d4.w);
+                const bool cont = p.bounce < p.max_bounces;
+                V3 c, so, sd;
+                float st, pl = 0.0f;
+                if (direct_light(p.sc, sf, thr, pix, p.sample, p.bounce, p.seed, p.epsilon, c, so, sd, st, &pl)) {
+                    if (p.mis && cont) c = c * power_weight(pl, bsdf_pdf(sf, sf.L));
+                    emitShadow = true;
+                    shRay0 = make_float4(so.x, so.y, so.z, __uint_as_float(pix));
+                    shRay1 = make_float4(sd.x, sd.y, sd.z, st);
+                    shPay = make_float4(c.x, c.y, c.z, __uint_as_float(pix));
+                }
+                if (cont) {
+                    V3 o, d;
+                    bool spec = false, passed = false;
+                    if (continue_path(sf, thr, pix, p.sample, p.bounce, p.seed, p.epsilon, o, d, &spec, &passed)) {
+                        emitRay = true;
+                        outRay0 = make_float4(o.x, o.y, o.z, __uint_as_float(pix));
+                        // a light seen through a pass-through is not part of the
+                        // engine's direct light (its NEE evaluates reflection only)
+                        outRay1 = make_float4(d.x, d.y, d.z,
+                                              p.mis && !passed ? mis_hit_factor(p.sc, sf, d, spec) : 0.0f);
+                        outPay = make_float4(thr.x, thr.y, thr.z, __uint_as_float(pix));
+                    }
                 }
             }
         }
-    }
-    uint32_t* const counters[2] = { p.n_out, p.n_shadow };
-    const bool want[2] = { emitRay, emitShadow };
-    uint32_t slot[2];
-    block_append<2>(counters, want, slot);
-    const uint32_t ri = slot[0], si = slot[1];
-    if (emitRay) {
-        float4* r = p.rays_out + size_t(ri) * 3;
-        r[0] = outRay0;
-        r[1] = outRay1;
-        r[2] = make_float4(0.0f, __int_as_float(-1), __int_as_float(-1), 0.0f);
-        p.pay_out[ri] = outPay;
-    }
-    if (emitShadow) {
-        float4* r = p.shadow_rays + size_t(si) * 3;
-        r[0] = shRay0;
-        r[1] = make_float4(shRay1.x, shRay1.y, shRay1.z, 0.0f);
-        r[2] = make_float4(shRay1.w, __int_as_float(-1), __int_as_float(-1), 0.0f);   // hit.x = tmax
-        p.shadow_pay[si] = shPay;
+        uint32_t* const counters[2] = { p.n_out, p.n_shadow };
+        const bool want[2] = { emitRay, emitShadow };
+        uint32_t slot[2];
+        block_append<2>(counters, want, slot);
+        const uint32_t ri = slot[0], si = slot[1];
+        if (emitRay) {
+            float4* r = p.rays_out + size_t(ri) * 3;
+            r[0] = outRay0;
+            r[1] = outRay1;
+            r[2] = make_float4(0.0f, __int_as_float(-1), __int_as_float(-1), 0.0f);
+            p.pay_out[ri] = outPay;
+        }
+        if (emitShadow) {
+            float4* r = p.shadow_rays + size_t(si) * 3;
+            r[0] = shRay0;
+            r[1] = make_float4(shRay1.x, shRay1.y, shRay1.z, 0.0f);
+            r[2] = make_float4(shRay1.w, __int_as_float(-1), __int_as_float(-1), 0.0f);   // hit.x = tmax
+            p.shadow_pay[si] = shPay;
+        }
     }
 }
 

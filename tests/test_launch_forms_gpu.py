@@ -200,3 +200,28 @@ def test_few_rays_on_a_context_of_one_cta_per_sm(few, n):
         assert np.array_equal(run({**few, "ctx": c, "mid": mid}, "any", n)[:n], few["full"]["any"][:n])
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("w,h", [(353, 276), (641, 479)])
+def test_path_tracer_queues_longer_than_the_shading_grid(w, h):
+    """A shading block that takes several chunks of its queue gives the image
+    of strips of which every block takes one; the 64-bit sums differ by the
+    order of at most 20 additions."""
+    import torch
+    from atlas_rt import ptscene
+    c = atlas_rt.Context(device=0)
+    try:
+        ptscene.upload(c, ptscene.build(seed=5, grid=64, n_boxes=20))
+        cam = atlas_rt.make_camera(scenes.pinhole_camera(w, h))
+        acc = torch.zeros((w * h, 4), device="cuda")
+        img = []
+        for rows in (h, 32):
+            acc64 = torch.zeros((w * h, 3), device="cuda", dtype=torch.float64)
+            for y in range(0, h, rows):
+                c.pathtrace(cam, acc, acc64, spp=2, tile=(0, y, w, min(rows, h - y)))
+            c.synchronize()
+            img.append(acc64.cpu().numpy())
+        np.testing.assert_allclose(img[0], img[1], rtol=20 * 2.0 ** -53, atol=0)
+        assert (img[0] > 0).mean() > 0.3
+    finally:
+        c.close()
