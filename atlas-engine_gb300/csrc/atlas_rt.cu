@@ -28,7 +28,7 @@ using atlas::rt::dev::TraceParams;
 // project's autotuner): warps per CTA and the shared-memory part of each
 // lane's 128-entry traversal stack (the rest spills to local memory).  The
 // register budget follows from the minimum resident CTAs per SM.
-constexpr int kStackEntries = 128;
+using atlas::rt::dev::kStackEntries;
 // Stack entries of the deep variants, launched for meshes and scenes whose
 // trees can need more than kStackEntries (local memory, 4 KB per lane).
 constexpr int kDeepStackEntries = 1024;
@@ -46,9 +46,9 @@ template <bool ANY, bool COUNT, int MODE, int W, int S, bool TIES = true, int ST
           int STACK = kStackEntries, bool CAMERA = false, bool FEW = false>
 void* KernelFor() {
     // 64 registers for 32 warps an SM; the scene kernels that detect near ties
-    // carry more per-lane state and get 72 (at 64: 1,892 against 1,842 us for
+    // carry more per-lane state and get 72 (at 64: 1,514 against 1,469 us for
     // the 512-instance scene; those without ties gain from 64, a path-traced
-    // sample 1,378 against 1,410 us).  36 or 40 warps of single-mesh kernels lose to
+    // sample 1,271 against 1,300 us).  36 or 40 warps of single-mesh kernels lose to
     // spills (1,126 against 1,074 us for a million random closest hits).
     constexpr bool wide = MODE == MODE_SCENE && TIES && !ANY;
     constexpr int minBlocks = wide ? (28 / W > 0 ? 28 / W : 1) : 32 / W;

@@ -225,3 +225,42 @@ def test_path_tracer_queues_longer_than_the_shading_grid(w, h):
         assert (img[0] > 0).mean() > 0.3
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("cap", [1, 2, 3, 4, 5, 9, 30, 0])
+@pytest.mark.parametrize("cull", [0xFFFFFFFF, 2])
+def test_scene_rounds_of_several_visits_keep_the_step_cap(cap, cull):
+    """Entering an instance and leaving a leaf visit the next node in the same
+    round unless the burst ends there: with bursts of one step they never do,
+    and every record and cap flag has to be the same."""
+    import torch
+    b = BVH(scenes.random_triangles(700, seed=21))
+    one = np.array([[[0, 0, 0], [1, 0, 0], [0, 1, 0]]], np.float32)
+    small = BVH(one.reshape(np.asarray(scenes.random_triangles(1, seed=1)).shape))
+    rays = torch.from_numpy(scenes.pack_rays(*scenes.sphere_rays(30000, seed=23))).cuda()
+    got = []
+    for burst in (1, 2, 24):
+        c = atlas_rt.Context(device=0, max_steps=cap, refill_steps=burst)
+        try:
+            ids = [c.upload_mesh(x.nodes, x.pack_triangles()) for x in (b, small)]
+            bounds = [atlas_rt.mesh_bounds(x) for x in (b, small)]
+            rng = np.random.default_rng(22)
+            inst, boxes = [], []
+            for i in range(24):
+                model = np.eye(4)
+                model[:3, :3] *= rng.uniform(0.2, 0.7)
+                model[:3, 3] = rng.uniform(-1.0, 1.0, 3)
+                inst.append(atlas_rt.make_instance(model, ids[i % 2], 1 + i % 3))
+                boxes.append(atlas_rt.transform_aabb(*bounds[i % 2], model))
+            c.scene_build(np.array(inst), np.array(boxes))
+            hits = torch.zeros((len(rays), 8), device="cuda")
+            occ = torch.zeros(len(rays), dtype=torch.uint8, device="cuda")
+            c.trace_scene_closest(rays, 1e-4, 10.0, cull_mask=cull, out=hits)
+            c.trace_scene_any(rays, 1e-4, 10.0, cull_mask=cull, out=occ)
+            torch.cuda.synchronize()
+            got.append((hits.cpu().numpy().view(np.uint32), occ.cpu().numpy()))
+        finally:
+            c.close()
+    for hits, occ in got[1:]:
+        assert np.array_equal(hits, got[0][0]) and np.array_equal(occ, got[0][1])
+    assert (got[0][0][:, 3] & atlas_rt.HIT_FLAG_ITER_CAP).any() == (0 < cap < 30) or cap == 30
