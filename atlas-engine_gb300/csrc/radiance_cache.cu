@@ -83,10 +83,13 @@ ae_rt_status Backprop(ae_rc* rc, const float4* recs, uint32_t n, const uint32_t*
                       uint32_t slices, cudaStream_t s, float* mlp_out = nullptr, float* grid_out = nullptr) {
     float* mlp = mlp_out ? mlp_out : rc->mlp_grad;
     float* grid = grid_out ? grid_out : rc->grid_grad;
-    if (mlp_out || !rc->grads_zero) RC_CUDA(rc, cudaMemsetAsync(mlp, 0, RC_NPARAM * sizeof(float), s));
-    if (grid_out || !rc->grads_zero) RC_CUDA(rc, cudaMemsetAsync(grid, 0, rc->grid_params * sizeof(float), s));
+    // whole 16-byte elements: 2^k of two floats at 16 levels, and RC_NPARAM
+    const uint32_t nm = mlp_out || !rc->grads_zero ? RC_NPARAM / 4 : 0;
+    const uint32_t ng = grid_out || !rc->grads_zero ? uint32_t(rc->grid_params / 4) : 0;
     if (!mlp_out || !grid_out) rc->grads_zero = false;
-    RC_CUDA(rc, cudaMemsetAsync(rc->d_loss, 0, sizeof(float), s));
+    rc_zero_kernel<<<ng ? uint32_t(rc->sm_count) : 1u, kZeroThreads, 0, s>>>(
+        reinterpret_cast<float4*>(grid), ng, reinterpret_cast<float4*>(mlp), nm, rc->d_loss);
+    RC_CUDA(rc, cudaGetLastError());
     RcMlpParams p = MlpParams(rc);
     p.grad_w = mlp;
     p.grid.grad = reinterpret_cast<float2*>(grid);
@@ -98,8 +101,19 @@ ae_rt_status Backprop(ae_rc* rc, const float4* recs, uint32_t n, const uint32_t*
     const uint32_t count = slices ? (n + slices - 1) / slices : n;
     if (rc->cfg.flags & AE_RC_TRAIN_WARP_MMA)
         rc_mlp_kernel<RC_TRAIN><<<GridBlocks(rc, count), RC_THREADS, kTrainSmem, s>>>(p);
-    else
-        rc_train_tc_kernel<<<GridBlocks(rc, count), RCTT_THREADS, RCTT_SMEM, s>>>(p);
+    else {
+        cudaLaunchAttribute overlap{};
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t launch{};
+        launch.gridDim = dim3(GridBlocks(rc, count));
+        launch.blockDim = dim3(RCTT_THREADS);
+        launch.dynamicSmemBytes = RCTT_SMEM;
+        launch.stream = s;
+        launch.attrs = &overlap;
+        launch.numAttrs = 1;
+        RC_CUDA(rc, cudaLaunchKernelEx(&launch, rc_train_tc_kernel, p));
+    }
     RC_CUDA(rc, cudaGetLastError());
     return AE_RT_OK;
 }
