@@ -319,7 +319,7 @@ ae_rt_status Launch(ae_rt_ctx* ctx, bool any, int mode, TraceParams& p, cudaStre
     if (!p.work_counter && !few_rays)
         AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     void* args[] = { &p };
-    AE_CUDA(ctx, cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, 0, s));
+    AE_CUDA(ctx, LaunchNext(static_cast<const void*>(fn), grid, threads, s, args));
     return AE_RT_OK;
 }
 
@@ -1259,8 +1259,7 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
         // ray generation into queue 0; it also sets the sample's counters
         p.rays_out = static_cast<float4*>(ctx->pt_rays[0].ptr);
         p.pay_out = static_cast<float4*>(ctx->pt_pay[0].ptr);
-        atlas::rt::dev::pt_raygen_kernel<<<blocks, 256, 0, s>>>(c, p);
-        AE_CUDA(ctx, cudaGetLastError());
+        AE_CUDA(ctx, LaunchNext(atlas::rt::dev::pt_raygen_kernel, blocks, 256, s, c, p));
         for (uint32_t b = 0; b <= params->max_bounces; b++) {
             const int in = int(b & 1), out = 1 - in, q = int(b & 1);
             p.bounce = b;
@@ -1286,8 +1285,8 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
             if (st != AE_RT_OK) return st;
             // this shadow queue's previous resolve must be done before it is refilled
             if (pending[q]) AE_CUDA(ctx, cudaStreamWaitEvent(s, ctx->pt_events[2 + q], 0));
-            atlas::rt::dev::pt_shade_kernel<<<shade_blocks, atlas::rt::dev::kShadeThreads, 0, s>>>(p);
-            AE_CUDA(ctx, cudaGetLastError());
+            AE_CUDA(ctx, LaunchNext(atlas::rt::dev::pt_shade_kernel, shade_blocks, atlas::rt::dev::kShadeThreads, s,
+                                    p));
             AE_CUDA(ctx, cudaEventRecord(ctx->pt_events[q], s));
             AE_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pt_events[q], 0));
             const ae_packed_ray* shadow_in = static_cast<const ae_packed_ray*>(shadowRays[q]->ptr);
@@ -1302,8 +1301,7 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
                            AE_RT_MASK_SHADOW, true, true, nullptr, w + 3);
             }
             if (st != AE_RT_OK) return st;
-            atlas::rt::dev::pt_resolve_kernel<<<blocks, 256, 0, side>>>(p);
-            AE_CUDA(ctx, cudaGetLastError());
+            AE_CUDA(ctx, LaunchNext(atlas::rt::dev::pt_resolve_kernel, blocks, 256, side, p));
             AE_CUDA(ctx, cudaEventRecord(ctx->pt_events[2 + q], side));
             pending[q] = true;
         }
@@ -1441,8 +1439,7 @@ ae_rt_status Spawn(ae_rt_ctx* ctx, int32_t mesh_id, const ae_packed_ray* rays, c
     sp.lightx = params->light_dir[0]; sp.lighty = params->light_dir[1]; sp.lightz = params->light_dir[2];
     sp.epsilon = params->epsilon;
     sp.seed = params->seed;
-    atlas::rt::dev::spawn_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(sp);
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(atlas::rt::dev::spawn_kernel, (n + 255) / 256, 256, static_cast<cudaStream_t>(stream), sp));
     return AE_RT_OK;
 }
 }  // namespace

@@ -151,6 +151,7 @@ __device__ __forceinline__ uint32_t block_append_sorted(uint32_t* counter, bool 
 }
 
 static __global__ void spawn_kernel(SpawnParams p) {
+    wait_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = p.n_dev ? min(*p.n_dev, p.n) : p.n;
     bool sec = false, shd = false;

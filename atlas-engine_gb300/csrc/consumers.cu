@@ -127,6 +127,7 @@ __device__ __forceinline__ V3 ggx_vndf_dir(V3 N, V3 V, float alpha, float u0, fl
 
 template <int KIND>
 __global__ void gb_raygen_kernel(GbParams g, PassP pp, Queue q, float* ao_out, float4* rad_out) {
+    wait_for_previous();
     const uint32_t n = g.w * g.h;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t pix = base + threadIdx.x;
@@ -240,6 +241,7 @@ struct DdgiP {
 // every warp 32 directions spread over the sphere).  Results still land at
 // probe * ray_count + i through the key.
 __global__ void ddgi_raygen_kernel(DdgiP d, Queue q) {
+    wait_for_previous();
     const uint32_t total = d.n_probes * d.ray_count;
     for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
         const uint32_t t = base + threadIdx.x;
@@ -277,6 +279,7 @@ __global__ void ddgi_raygen_kernel(DdgiP d, Queue q) {
 
 // RTAO output: ao = 1 - occlusion (rtao.csh:93-106)
 __global__ void ao_resolve_kernel(Queue q, const uint8_t* occ, const float* transparency, float* ao_out) {
+    wait_for_previous();
     const uint32_t n = min(*q.count, q.capacity);
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const float hit = transparency ? __fsub_rn(1.0f, transparency[e]) : (occ[e] ? 1.0f : 0.0f);
@@ -298,6 +301,7 @@ struct ShadeP {
 // GI) and ddgi/rayHit.csh:62-95 (DDGI), up to the visibility test.
 template <int KIND>
 __global__ void pass_shade_kernel(ShadeP p) {
+    wait_for_previous();
     const uint32_t n = min(*p.q.count, p.q.capacity);
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t e = base + threadIdx.x;
@@ -356,6 +360,7 @@ __global__ void pass_shade_kernel(ShadeP p) {
 // the light a shadow ray carries, times its visibility
 __global__ void pass_shadow_resolve_kernel(Queue sq, const float4* shadow_pay, const uint8_t* occ,
                                            const float* transparency, float4* rad) {
+    wait_for_previous();
     const uint32_t n = min(*sq.count, sq.capacity);
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const float vis = transparency ? transparency[s] : (occ[s] ? 0.0f : 1.0f);
@@ -372,6 +377,7 @@ __device__ __forceinline__ uint32_t half_bits(float x) { return __half_as_ushort
 
 template <int KIND>
 __global__ void pass_output_kernel(Queue q, const float4* rad, float limit, float4* out) {
+    wait_for_previous();
     const uint32_t n = min(*q.count, q.capacity);
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const float4 r = rad[e];
@@ -513,8 +519,7 @@ ae_rt_status ShadeAndResolve(ae_rt_ctx* ctx, const PassP& pp, const Queue& q, co
     sp.sq = sq;
     sp.shadow_pay = static_cast<float4*>(ctx->pass_shadow_pay.ptr);
     const uint32_t blocks = Blocks(ctx, q.capacity);
-    pass_shade_kernel<KIND><<<blocks, 256, 0, s>>>(sp);
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(pass_shade_kernel<KIND>, blocks, 256, s, sp));
     const ae_packed_ray* srays = reinterpret_cast<const ae_packed_ray*>(sq.rays);
     ae_rt_status st;
     if (KIND == kPassDDGI)   // CheckVisibility, ddgi/rayHit.csh:140-151
@@ -525,12 +530,11 @@ ae_rt_status ShadeAndResolve(ae_rt_ctx* ctx, const PassP& pp, const Queue& q, co
                                sq.count, true);
     if (st != AE_RT_OK) return st;
     const bool opaqueVis = KIND == kPassDDGI;
-    pass_shadow_resolve_kernel<<<blocks, 256, 0, s>>>(
-        sq, sp.shadow_pay, opaqueVis ? static_cast<const uint8_t*>(ctx->pass_vis.ptr) : nullptr,
-        opaqueVis ? nullptr : static_cast<const float*>(ctx->pass_vis.ptr), sp.rad);
-    AE_CUDA(ctx, cudaGetLastError());
-    pass_output_kernel<KIND><<<blocks, 256, 0, s>>>(q, sp.rad, pp.limit, out);
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(
+        pass_shadow_resolve_kernel, blocks, 256, s, sq, sp.shadow_pay,
+        opaqueVis ? static_cast<const uint8_t*>(ctx->pass_vis.ptr) : nullptr,
+        opaqueVis ? nullptr : static_cast<const float*>(ctx->pass_vis.ptr), sp.rad));
+    AE_CUDA(ctx, LaunchNext(pass_output_kernel<KIND>, blocks, 256, s, q, sp.rad, pp.limit, out));
     return AE_RT_OK;
 }
 
@@ -553,16 +557,14 @@ ae_rt_status ScreenPass(ae_rt_ctx* ctx, const ae_gbuffer* gb, const ae_rt_pass_p
     AE_CUDA(ctx, cudaMemsetAsync(q.count, 0, 2 * sizeof(uint32_t), s));
     const PassP pp = Pass(params);
     const bool opacity = (params->flags & AE_PASS_OPACITY_CHECK) != 0;
-    gb_raygen_kernel<KIND><<<Blocks(ctx, n), 256, 0, s>>>(GBuffer(gb), pp, q, static_cast<float*>(out),
-                                                          static_cast<float4*>(out));
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(gb_raygen_kernel<KIND>, Blocks(ctx, n), 256, s, GBuffer(gb), pp, q,
+                            static_cast<float*>(out), static_cast<float4*>(out)));
     if (KIND == kPassAO) {
         st = TracePrimary(ctx, true, opacity, q, params->radius, ctx->pass_vis.ptr, stream);
         if (st != AE_RT_OK) return st;
-        ao_resolve_kernel<<<Blocks(ctx, n), 256, 0, s>>>(
-            q, opacity ? nullptr : static_cast<const uint8_t*>(ctx->pass_vis.ptr),
-            opacity ? static_cast<const float*>(ctx->pass_vis.ptr) : nullptr, static_cast<float*>(out));
-        AE_CUDA(ctx, cudaGetLastError());
+        AE_CUDA(ctx, LaunchNext(
+            ao_resolve_kernel, Blocks(ctx, n), 256, s, q, opacity ? nullptr : static_cast<const uint8_t*>(ctx->pass_vis.ptr),
+            opacity ? static_cast<const float*>(ctx->pass_vis.ptr) : nullptr, static_cast<float*>(out)));
         return AE_RT_OK;
     }
     st = TracePrimary(ctx, false, opacity, q, kInfT, ctx->pass_hits.ptr, stream);
@@ -618,8 +620,7 @@ ae_rt_status ae_rt_ddgi_trace(ae_rt_ctx* ctx, const ae_ddgi_probes* probes, cons
     d.ray_count = probes->ray_count;
     d.inactive_count = probes->inactive_ray_count < probes->ray_count ? probes->inactive_ray_count
                                                                      : probes->ray_count;
-    ddgi_raygen_kernel<<<Blocks(ctx, uint32_t(total)), 256, 0, s>>>(d, q);
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(ddgi_raygen_kernel, Blocks(ctx, uint32_t(total)), 256, s, d, q));
     const bool opacity = (params->flags & AE_PASS_OPACITY_CHECK) != 0;
     st = TracePrimary(ctx, false, opacity, q, kInfT, ctx->pass_hits.ptr, stream);
     if (st != AE_RT_OK) return st;

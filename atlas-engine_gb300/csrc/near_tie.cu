@@ -187,6 +187,7 @@ __global__ void retest_compact_kernel(RetestParams p) {
 // takes no double-precision operation.
 __global__ void __launch_bounds__(kRetestThreads, kRetestBlocks) retest_kernel(RetestParams p) {
     using namespace atlas::rt::dev;
+    wait_for_previous();
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ int32_t s_stack[kRetestThreads / 32][kRetestSmem][32];
     const uint32_t count = *p.n_retested;
@@ -370,8 +371,7 @@ extern "C" ae_rt_status ae_rt_retest_near_ties(ae_rt_ctx* ctx, int32_t mesh_id, 
     const uint32_t warps_per_block = kRetestThreads / 32;
     const uint32_t cap2 = uint32_t(ctx->sm_count) * uint32_t(kRetestBlocks);
     const uint32_t blocks2 = std::min((n_rays + warps_per_block - 1) / warps_per_block, cap2);
-    retest_kernel<<<blocks2, kRetestThreads, 0, s>>>(p);
-    AE_CUDA(ctx, cudaGetLastError());
+    AE_CUDA(ctx, LaunchNext(retest_kernel, blocks2, kRetestThreads, s, p));
     if (n_retested) {
         AE_CUDA(ctx, cudaMemcpyAsync(n_retested, p.n_retested, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         return ae_rt_synchronize(ctx, stream);

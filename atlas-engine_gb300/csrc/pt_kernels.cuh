@@ -347,6 +347,7 @@ __device__ __forceinline__ Light load_light(const float4* l) {
 }
 
 static __global__ void pt_raygen_kernel(CameraParams c, PtParams p) {
+    wait_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = p.tile_w * p.tile_h;
     if (i >= n) return;
@@ -804,6 +805,7 @@ constexpr uint32_t kShadeCtas = 5;
 // chunks of a persistent grid).  Bound by instruction issue and by the latency
 // of the triangle's and the material's dependent loads.
 static __global__ void __launch_bounds__(kShadeThreads, kShadeCtas) pt_shade_kernel(PtParams p) {
+    wait_for_previous();
     __shared__ uint32_t s_hits[kShadeThreads / 32];
     __shared__ uint32_t s_item[2 * kShadeThreads];   // hits waiting to be shaded
     const uint32_t n = min(*p.n_in, queue_capacity(p));
@@ -912,6 +914,7 @@ static __global__ void __launch_bounds__(kShadeThreads, kShadeCtas) pt_shade_ker
 
 // Adds the contributions of the unoccluded shadow rays.
 static __global__ void pt_resolve_kernel(PtParams p) {
+    wait_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = min(*p.n_shadow, queue_capacity(p));
     if (i >= n) return;

@@ -168,6 +168,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // pointer of a valid tree (arrays hold fewer than 2^31 - 1 elements).
 constexpr int32_t kStackEnd = INT32_MIN;
 
+// First statement of every kernel that host::LaunchNext launches: such a
+// kernel is set up while the one before it on the stream drains, and this
+// waits until that has ended and its writes are visible.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Stack entries of a lane; meshes and scenes whose trees can need more take
 // kernels with a deeper stack.
 constexpr int kStackEntries = 128;
@@ -1165,6 +1170,7 @@ template <bool ANY, bool COUNT, int MODE, int WARPS, int SMEM_STACK, int SPILL_S
           bool BOUNDS = false, bool TIES = true, int STAGE = 0, bool LOOSE = false, bool CAMERA = false,
           bool OPACITY = false, bool FEW = false>
 __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS) trace_kernel(TraceParams p) {
+    wait_for_previous();
     trace_rays<ANY, COUNT, MODE, WARPS, SMEM_STACK, SPILL_STACK, BOUNDS, TIES, STAGE, LOOSE, CAMERA, OPACITY, FEW>(p);
 }
 

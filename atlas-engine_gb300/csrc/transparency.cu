@@ -89,7 +89,7 @@ ae_rt_status atlas::rt::host::TraceTransparency(ae_rt_ctx* ctx, bool any, const 
     void* fn = any ? (shallow ? KernelFor<true, 0>() : KernelFor<true, 96>())
                    : (shallow ? KernelFor<false, 0>() : KernelFor<false, 96>());
     void* args[] = { &p };
-    AE_CUDA(ctx, cudaLaunchKernel(fn, dim3(GridFor(ctx, fn, n, 128)), dim3(128), args, 0, s));
+    AE_CUDA(ctx, LaunchNext(static_cast<const void*>(fn), GridFor(ctx, fn, n, 128), 128, s, args));
     if (!out_dev) AE_CUDA(ctx, cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, s));
     if (!out_dev || !rays_dev) return ae_rt_synchronize(ctx, stream);
     return AE_RT_OK;
