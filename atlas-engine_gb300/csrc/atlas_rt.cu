@@ -446,9 +446,10 @@ ae_rt_status atlas::rt::host::EnsureBounceQueues(ae_rt_ctx* ctx, uint32_t capaci
 
 ae_rt_status atlas::rt::host::TraceSceneQueue(ae_rt_ctx* ctx, bool any, const ae_packed_ray* rays, uint32_t capacity,
                                              float tmin, float tmax, void* out, void* stream,
-                                             const uint32_t* count_dev, uint32_t cull_mask, bool per_ray_tmax) {
+                                             const uint32_t* count_dev, uint32_t cull_mask, bool per_ray_tmax,
+                                             uint32_t* counter) {
     return Trace(ctx, any, kSceneTarget, rays, capacity, tmin, tmax, out, stream, count_dev, cull_mask, per_ray_tmax,
-                 false);
+                 false, nullptr, counter);
 }
 
 namespace {

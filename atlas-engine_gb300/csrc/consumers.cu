@@ -14,7 +14,7 @@
 //      and append one shadow ray per lit hit to a second queue;
 //   4. the shadow trace (HitAnyTransparency for reflections and GI,
 //      HitAny for DDGI, mask SHADOW, per-ray tmax = light distance -
-//      2 EPSILON), a resolve that adds the visible light, and the output
+//      2 EPSILON), and the output with the visible light added
 //      (radiance limit, or PackRayHit for DDGI).
 // Random numbers: the caller's per-pixel samples (the shaders' blue-noise
 // vector) where given, else the PCG hash of (pixel, frame_seed); light
@@ -287,6 +287,8 @@ __global__ void ao_resolve_kernel(Queue q, const uint8_t* occ, const float* tran
     }
 }
 
+constexpr uint32_t kNoShadow = 0xffffffffu;
+
 struct ShadeP {
     PtScene sc;
     PassP pp;
@@ -294,7 +296,7 @@ struct ShadeP {
     const float4* hits;      // ae_hit per queue entry
     float4* rad;             // per queue entry: radiance so far, hit distance
     Queue sq;                // shadow rays
-    float4* shadow_pay;      // per shadow ray: contribution, primary entry
+    float4* light;           // per queue entry: contribution and slot of its shadow ray (kNoShadow: none)
 };
 
 // EvaluateHit of rtreflection.csh:152-182 / rtgi.csh:155-185 (reflections,
@@ -334,7 +336,7 @@ __global__ void pass_shade_kernel(ShadeP p) {
                             sr0 = make_float4(so.x, so.y, so.z, 0.0f);
                             sr1 = make_float4(sf.L.x, sf.L.y, sf.L.z, 0.0f);
                             sr2 = make_float4(ls.dist - 2.0f * kEps, __int_as_float(-1), __int_as_float(-1), 0.0f);
-                            pay = make_float4(c.x, c.y, c.z, __uint_as_float(e));
+                            pay = make_float4(c.x, c.y, c.z, 0.0f);
                             emit = true;
                         }
                     }
@@ -347,40 +349,46 @@ __global__ void pass_shade_kernel(ShadeP p) {
         uint32_t slots[1];
         block_append<1>(counters, want, slots);
         const uint32_t slot = slots[0];
-        if (emit && slot < p.sq.capacity) {
+        emit = emit && slot < p.sq.capacity;
+        if (emit) {
             float4* r = p.sq.rays + size_t(slot) * 3;
             r[0] = sr0;
             r[1] = sr1;
             r[2] = sr2;
-            p.shadow_pay[slot] = pay;
         }
-    }
-}
-
-// the light a shadow ray carries, times its visibility
-__global__ void pass_shadow_resolve_kernel(Queue sq, const float4* shadow_pay, const uint8_t* occ,
-                                           const float* transparency, float4* rad) {
-    wait_for_previous();
-    const uint32_t n = min(*sq.count, sq.capacity);
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const float vis = transparency ? transparency[s] : (occ[s] ? 0.0f : 1.0f);
-        if (vis == 0.0f) continue;
-        const float4 c = shadow_pay[s];
-        float4& r = rad[__float_as_uint(c.w)];
-        r.x += c.x * vis;
-        r.y += c.y * vis;
-        r.z += c.z * vis;
+        if (e < n) {
+            pay.w = __uint_as_float(emit ? slot : kNoShadow);
+            p.light[e] = pay;
+        }
     }
 }
 
 __device__ __forceinline__ uint32_t half_bits(float x) { return __half_as_ushort(__float2half_rn(x)); }
 
+// An entry's radiance with the light of its shadow ray where that is visible,
+// in the pass's output format.  (Adding the light in a kernel of its own, a
+// thread per shadow ray, took another pass over `rad` and a launch; with the
+// two work counters' clears the four passes took 1,013 against 989 us.)
+// visible: what the shadow rays' trace wrote, occlusion bytes (DDGI) or
+// transparencies.
 template <int KIND>
-__global__ void pass_output_kernel(Queue q, const float4* rad, float limit, float4* out) {
+__global__ void pass_output_kernel(Queue q, const float4* rad, const float4* light, const void* visible, float limit,
+                                   float4* out) {
     wait_for_previous();
     const uint32_t n = min(*q.count, q.capacity);
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const float4 r = rad[e];
+        float4 r = rad[e];
+        const float4 c = light[e];
+        const uint32_t slot = __float_as_uint(c.w);
+        float vis = 0.0f;
+        if (slot != kNoShadow)
+            vis = KIND == kPassDDGI ? (static_cast<const uint8_t*>(visible)[slot] ? 0.0f : 1.0f)
+                                    : static_cast<const float*>(visible)[slot];
+        if (vis != 0.0f) {
+            r.x += c.x * vis;
+            r.y += c.y * vis;
+            r.z += c.z * vis;
+        }
         if (KIND == kPassDDGI) {
             // PackRayHit, ddgi/ddgi.hsh:85-98
             const float4 d = q.rays[size_t(e) * 3 + 1];
@@ -480,6 +488,11 @@ GbParams GBuffer(const ae_gbuffer* gb) {
     return g;
 }
 
+// pass_counts: the queues' lengths and the work counters of the pass's two
+// traces, cleared by one operation at its start (a memset before each trace
+// was an operation of its own between two kernels).
+constexpr uint32_t kPassWords = 4;
+
 // Scratch of the passes for `cap` primary rays: queue, hits, per-entry
 // radiance, shadow queue.
 ae_rt_status EnsurePassScratch(ae_rt_ctx* ctx, uint32_t cap, Queue& q, Queue& sq) {
@@ -490,7 +503,7 @@ ae_rt_status EnsurePassScratch(ae_rt_ctx* ctx, uint32_t cap, Queue& q, Queue& sq
     AE_CUDA(ctx, ctx->pass_shadow.ensure(size_t(cap) * sizeof(ae_packed_ray)));
     AE_CUDA(ctx, ctx->pass_shadow_pay.ensure(size_t(cap) * sizeof(float4)));
     AE_CUDA(ctx, ctx->pass_vis.ensure(size_t(cap) * sizeof(float)));
-    AE_CUDA(ctx, ctx->pass_counts.ensure(2 * sizeof(uint32_t)));
+    AE_CUDA(ctx, ctx->pass_counts.ensure(kPassWords * sizeof(uint32_t)));
     uint32_t* counts = static_cast<uint32_t*>(ctx->pass_counts.ptr);
     q = Queue{ static_cast<float4*>(ctx->pass_rays.ptr), static_cast<uint32_t*>(ctx->pass_key.ptr), counts, cap };
     sq = Queue{ static_cast<float4*>(ctx->pass_shadow.ptr), nullptr, counts + 1, cap };
@@ -501,11 +514,14 @@ ae_rt_status EnsurePassScratch(ae_rt_ctx* ctx, uint32_t cap, Queue& q, Queue& sq
 ae_rt_status TracePrimary(ae_rt_ctx* ctx, bool any, bool opacity, const Queue& q, float tmax, void* out,
                           void* stream) {
     const ae_packed_ray* rays = reinterpret_cast<const ae_packed_ray*>(q.rays);
-    if (opacity) return TraceTransparency(ctx, any, rays, q.capacity, 0.0f, tmax, AE_RT_MASK_ALL, out, stream, q.count);
-    return TraceSceneQueue(ctx, any, rays, q.capacity, 0.0f, tmax, out, stream, q.count, AE_RT_MASK_ALL, false);
+    if (opacity)
+        return TraceTransparency(ctx, any, rays, q.capacity, 0.0f, tmax, AE_RT_MASK_ALL, out, stream, q.count, false,
+                                 q.count + 2);
+    return TraceSceneQueue(ctx, any, rays, q.capacity, 0.0f, tmax, out, stream, q.count, AE_RT_MASK_ALL, false,
+                           q.count + 2);
 }
 
-// Steps 3-4 of the shading passes: shade, shadow trace, resolve, output.
+// Steps 3-4 of the shading passes: shade, shadow trace, output.
 template <int KIND>
 ae_rt_status ShadeAndResolve(ae_rt_ctx* ctx, const PassP& pp, const Queue& q, const Queue& sq, float4* out,
                              cudaStream_t s) {
@@ -517,24 +533,20 @@ ae_rt_status ShadeAndResolve(ae_rt_ctx* ctx, const PassP& pp, const Queue& q, co
     sp.hits = static_cast<const float4*>(ctx->pass_hits.ptr);
     sp.rad = static_cast<float4*>(ctx->pass_rad.ptr);
     sp.sq = sq;
-    sp.shadow_pay = static_cast<float4*>(ctx->pass_shadow_pay.ptr);
+    sp.light = static_cast<float4*>(ctx->pass_shadow_pay.ptr);
     const uint32_t blocks = Blocks(ctx, q.capacity);
     AE_CUDA(ctx, LaunchNext(pass_shade_kernel<KIND>, blocks, 256, s, sp));
     const ae_packed_ray* srays = reinterpret_cast<const ae_packed_ray*>(sq.rays);
     ae_rt_status st;
     if (KIND == kPassDDGI)   // CheckVisibility, ddgi/rayHit.csh:140-151
         st = TraceSceneQueue(ctx, true, srays, sq.capacity, 0.0f, kInfT, ctx->pass_vis.ptr, s, sq.count,
-                             AE_RT_MASK_SHADOW, true);
+                             AE_RT_MASK_SHADOW, true, q.count + 3);
     else                     // CheckVisibility, rtreflection.csh:232-245 / rtgi.csh:222-234
         st = TraceTransparency(ctx, true, srays, sq.capacity, 0.0f, kInfT, AE_RT_MASK_SHADOW, ctx->pass_vis.ptr, s,
-                               sq.count, true);
+                               sq.count, true, q.count + 3);
     if (st != AE_RT_OK) return st;
-    const bool opaqueVis = KIND == kPassDDGI;
-    AE_CUDA(ctx, LaunchNext(
-        pass_shadow_resolve_kernel, blocks, 256, s, sq, sp.shadow_pay,
-        opaqueVis ? static_cast<const uint8_t*>(ctx->pass_vis.ptr) : nullptr,
-        opaqueVis ? nullptr : static_cast<const float*>(ctx->pass_vis.ptr), sp.rad));
-    AE_CUDA(ctx, LaunchNext(pass_output_kernel<KIND>, blocks, 256, s, q, sp.rad, pp.limit, out));
+    AE_CUDA(ctx, LaunchNext(pass_output_kernel<KIND>, blocks, 256, s, q, sp.rad, sp.light, ctx->pass_vis.ptr, pp.limit,
+                            out));
     return AE_RT_OK;
 }
 
@@ -554,7 +566,7 @@ ae_rt_status ScreenPass(ae_rt_ctx* ctx, const ae_gbuffer* gb, const ae_rt_pass_p
     Queue q, sq;
     st = EnsurePassScratch(ctx, n, q, sq);
     if (st != AE_RT_OK) return st;
-    AE_CUDA(ctx, cudaMemsetAsync(q.count, 0, 2 * sizeof(uint32_t), s));
+    AE_CUDA(ctx, cudaMemsetAsync(q.count, 0, kPassWords * sizeof(uint32_t), s));
     const PassP pp = Pass(params);
     const bool opacity = (params->flags & AE_PASS_OPACITY_CHECK) != 0;
     AE_CUDA(ctx, LaunchNext(gb_raygen_kernel<KIND>, Blocks(ctx, n), 256, s, GBuffer(gb), pp, q,
@@ -609,7 +621,7 @@ ae_rt_status ae_rt_ddgi_trace(ae_rt_ctx* ctx, const ae_ddgi_probes* probes, cons
     Queue q, sq;
     st = EnsurePassScratch(ctx, uint32_t(total), q, sq);
     if (st != AE_RT_OK) return st;
-    AE_CUDA(ctx, cudaMemsetAsync(q.count, 0, 2 * sizeof(uint32_t), s));
+    AE_CUDA(ctx, cudaMemsetAsync(q.count, 0, kPassWords * sizeof(uint32_t), s));
     DdgiP d{};
     d.probes = reinterpret_cast<const float4*>(probes->probes);
     d.dirs = reinterpret_cast<const float4*>(probes->ray_dirs);

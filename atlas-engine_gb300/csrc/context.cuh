@@ -207,10 +207,11 @@ uint32_t SpreadWarps(const ae_rt_ctx* ctx);
 // Queue-driven trace over the context's two-level scene (rays, out and count
 // in device memory), for the other translation units.
 // Closest / any-hit trace of a scene queue for the library's own consumers
-// (passes, radiance cache): the near-tie detection is skipped.
+// (passes, radiance cache): the near-tie detection is skipped; counter: a work
+// counter that an earlier operation on the stream zeroed, or null.
 ae_rt_status TraceSceneQueue(ae_rt_ctx* ctx, bool any, const ae_packed_ray* rays, uint32_t capacity, float tmin,
                              float tmax, void* out, void* stream, const uint32_t* count_dev, uint32_t cull_mask,
-                             bool per_ray_tmax);
+                             bool per_ray_tmax, uint32_t* counter = nullptr);
 
 // The transparency traversal variants over the scene (transparency.cu); with
 // count_dev, `n` is the queue capacity and the count lives on the device;

@@ -264,3 +264,57 @@ def test_scene_rounds_of_several_visits_keep_the_step_cap(cap, cull):
     for hits, occ in got[1:]:
         assert np.array_equal(hits, got[0][0]) and np.array_equal(occ, got[0][1])
     assert (got[0][0][:, 3] & atlas_rt.HIT_FLAG_ITER_CAP).any() == (0 < cap < 30) or cap == 30
+
+
+@pytest.mark.parametrize("kind", ["closest", "any", "scene", "pathtrace", "passes"])
+def test_chained_launches_in_a_captured_graph(few, kind):
+    """Chains of launches that are set up ahead of the previous one's end,
+    recorded once and replayed twice over cleared outputs: the eager results."""
+    import torch
+    from atlas_rt import gbuffer, ptscene
+    c = few["ctx"]
+    if kind in ("pathtrace", "passes"):
+        c = atlas_rt.Context(device=0)
+        _, shading, _, _ = ptscene.upload(c, ptscene.build(seed=3, grid=24, n_boxes=8))
+    try:
+        w, h = 97, 65
+        hits = torch.zeros((len(few["rays"]), 8), device="cuda")
+        occ = torch.zeros(len(few["rays"]), dtype=torch.uint8, device="cuda")
+        image, gi = torch.zeros((w * h, 4), device="cuda"), torch.zeros((h, w, 4), device="cuda")
+        outs = [hits, occ, image, gi]
+        cam = atlas_rt.make_camera(scenes.pinhole_camera(w, h))
+        if kind == "passes":
+            view = gbuffer.look_at((50.0, 30.0, -40.0), (50.0, 0.0, 50.0))
+            gb = gbuffer.device_gbuffer(c, shading, view, gbuffer.perspective(60.0, w / h, 0.5, 400.0), w, h)
+
+        def chain(stream):
+            for _ in range(2):
+                if kind == "closest":
+                    c.trace_closest(few["mid"], few["rays"], 1e-4, 10.0, out=hits, stream=stream)
+                elif kind == "any":
+                    c.trace_any(few["mid"], few["rays"], 1e-4, 10.0, out=occ, stream=stream)
+                elif kind == "scene":
+                    c.trace_scene_closest(few["rays"], 1e-4, 10.0, out=hits, stream=stream)
+                elif kind == "pathtrace":
+                    c.pathtrace(cam, image, spp=1, stream=stream)
+                else:
+                    c.rtgi(gb, gi, frame_seed=5, stream=stream)
+
+        side = torch.cuda.Stream()
+        chain(side.cuda_stream)
+        side.synchronize()
+        want = [o.cpu().numpy().view(np.uint8).copy() for o in outs]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            for o in outs:
+                o.zero_()
+            chain(side.cuda_stream)
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        for o, v in zip(outs, want):
+            assert np.array_equal(o.cpu().numpy().view(np.uint8), v)
+        assert any(v.any() for v in want)
+    finally:
+        if c is not few["ctx"]:
+            c.close()
