@@ -146,7 +146,7 @@ __device__ __forceinline__ bool same_triangle(const float4* q, const float4& A, 
 
 // Pass 1: every ray's result as the FP32 trace left it, and the list of the
 // flagged rays (warp-aggregated appends), so that the double-precision pass
-// runs one flagged ray per thread with full warps.
+// spreads them evenly over its warps.
 __global__ void retest_compact_kernel(RetestParams p) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     const size_t n_iter = (size_t(p.n) + stride - 1) / stride * stride;
