@@ -318,3 +318,37 @@ def test_chained_launches_in_a_captured_graph(few, kind):
     finally:
         if c is not few["ctx"]:
             c.close()
+
+
+@pytest.mark.parametrize("w,h", [(17, 3), (641, 479), (1201, 701)])
+def test_pass_queues_longer_than_the_shading_grid(w, h):
+    """Reflections and GI of a frame whose shading blocks take several chunks
+    of the queue, against the same frame with all but 96 rows at the far plane
+    at a time, of whose queue every block takes one: samples are keyed by the
+    pixel, so the bits are the same."""
+    import torch
+    from atlas_rt import gbuffer, ptscene
+    c = atlas_rt.Context(device=0)
+    try:
+        _, shading, _, _ = ptscene.upload(c, ptscene.build(seed=9, grid=48, n_boxes=20))
+        view = gbuffer.look_at((50.0, 30.0, -40.0), (50.0, 0.0, 50.0))
+        gb = gbuffer.device_gbuffer(c, shading, view, gbuffer.perspective(60.0, w / h, 0.5, 400.0), w, h)
+        gb["roughness"] = torch.full((h, w), 0.4, device="cuda")
+        depth = gb["depth"].reshape(h, w).clone()
+        full, part = torch.zeros((h, w, 4), device="cuda"), torch.zeros((h, w, 4), device="cuda")
+        lit = 0.0
+        for run in (c.rtgi, c.reflections):
+            gb["depth"] = depth
+            run(gb, full, frame_seed=5)
+            for y in range(0, h, 96):
+                gb["depth"] = torch.ones_like(depth)
+                gb["depth"][y:y + 96] = depth[y:y + 96]
+                run(gb, part, frame_seed=5)
+                c.synchronize()
+                assert torch.equal(part[y:y + 96].view(torch.int32), full[y:y + 96].view(torch.int32))
+            lit += float(full[..., :3].sum())
+        assert lit > 0
+        # the largest frame's queue is longer than eight blocks of 128 an SM
+        assert (int((depth < 1).sum()) > 8 * 128 * 152) == (w > 1000)
+    finally:
+        c.close()
