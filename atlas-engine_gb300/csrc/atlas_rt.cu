@@ -1243,6 +1243,7 @@ ae_rt_status PathTrace(ae_rt_ctx* ctx, const ae_camera* cam, const ae_pt_params*
     p.n_words = 4 * uint32_t(std::min<uint64_t>(uint64_t(params->max_bounces) + 2, kWordSets));
     AE_CUDA(ctx, ctx->pt_words.ensure(p.n_words * sizeof(uint32_t)));
     p.words = static_cast<uint32_t*>(ctx->pt_words.ptr);
+    p.overflow = ctx->d_counter + 1;
     const float kInf = 1e12f;   // INF of common.hsh:8
     // Shadow queues alternate between two buffers: a bounce's shadow trace and
     // resolve run on the side stream while the next bounce is traced and shaded

@@ -350,6 +350,10 @@ static __global__ void pt_raygen_kernel(CameraParams c, PtParams p) {
     wait_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = p.tile_w * p.tile_h;
+    // the sample's counters: this queue's length, zeros for everything after
+    // it; by every thread of the block, also those past a small tile's pixels
+    if (p.words && blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < p.n_words; k += blockDim.x) p.words[k] = k == 0 ? n : 0u;
     if (i >= n) return;
     const uint32_t t = slot_to_pixel(i, p.tile_w, p.tile_h);
     const uint32_t px = p.tile_x0 + t % p.tile_w, py = p.tile_y0 + t / p.tile_w;
@@ -370,13 +374,7 @@ static __global__ void pt_raygen_kernel(CameraParams c, PtParams p) {
     r[1] = make_float4(d.x, d.y, d.z, 0.0f);
     r[2] = make_float4(0.0f, __int_as_float(-1), __int_as_float(-1), 0.0f);
     p.pay_out[i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(pix));
-    if (p.words) {
-        // the sample's counters: this queue's length, zeros for everything after it
-        if (blockIdx.x == 0)
-            for (uint32_t k = threadIdx.x; k < p.n_words; k += blockDim.x) p.words[k] = k == 0 ? n : 0u;
-    } else if (i == 0) {
-        *p.n_out = n;
-    }
+    if (!p.words && i == 0) *p.n_out = n;
 }
 
 __device__ __forceinline__ void add_radiance(const PtParams& p, uint32_t key, V3 L) {
@@ -894,15 +892,16 @@ static __global__ void __launch_bounds__(kShadeThreads, kShadeCtas) pt_shade_ker
         const bool want[2] = { emitRay, emitShadow };
         uint32_t slot[2];
         block_append<2>(counters, want, slot);
-        const uint32_t ri = slot[0], si = slot[1];
-        if (emitRay) {
+        const uint32_t ri = slot[0], si = slot[1], cap = queue_capacity(p);
+        if (p.overflow && ((emitRay && ri >= cap) || (emitShadow && si >= cap))) atomicOr(p.overflow, kErrQueueOverflow);
+        if (emitRay && ri < cap) {
             float4* r = p.rays_out + size_t(ri) * 3;
             r[0] = outRay0;
             r[1] = outRay1;
             r[2] = make_float4(0.0f, __int_as_float(-1), __int_as_float(-1), 0.0f);
             p.pay_out[ri] = outPay;
         }
-        if (emitShadow) {
+        if (emitShadow && si < cap) {
             float4* r = p.shadow_rays + size_t(si) * 3;
             r[0] = shRay0;
             r[1] = make_float4(shRay1.x, shRay1.y, shRay1.z, 0.0f);
