@@ -455,9 +455,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // The gradients' and the loss's zeros, written while the training kernel
 // launched behind it (programmatic dependent launch) sets up, gathers and runs
 // its first tile forward; that kernel waits (rc_zeros_done) before it adds to
-// any of them.  One block of 256 threads an SM: its 4 K registers fit beside a
-// training CTA's 61 K.  With three memsets before an ordinary launch the
-// gradients of 65,536 records at 2^19 entries a level took 121 us, this way 106.
+// any of them, and every thread of it before it ends.  One block of 256 threads
+// an SM: its 4 K registers fit beside a training CTA's 61 K.  With three
+// memsets before an ordinary launch the gradients of 65,536 records at 2^19
+// entries a level took 121 us, this way 106.
 constexpr uint32_t kZeroThreads = 256;
 static __global__ void __launch_bounds__(kZeroThreads) rc_zero_kernel(float4* a, uint32_t na, float4* b, uint32_t nb,
                                                                       float* loss) {
@@ -746,6 +747,9 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
             }
         }
     }
+    // also where no tile was, or a wait gave up: the kernel behind this one
+    // starts when this grid has ended, and reads what the zeros went into
+    rc_zeros_done();
     tc_fence_before();
     __syncthreads();
     if (*fail && tid == 0 && p.error_word) atomicOr(p.error_word, kErrTimeout);
