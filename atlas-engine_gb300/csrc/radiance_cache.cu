@@ -553,14 +553,20 @@ ae_rt_status ae_rc_selftest_wait_timeout(ae_rc* rc, uint32_t* timed_out) {
     p.n = RCT_THREADS;
     p.out = out;
     p.skip_mma = 1;
-    rc_infer_tc_kernel<RC_PREDICT><<<1, RCT_THREADS, RCT_SMEM>>>(p);
-    cudaError_t e = cudaGetLastError();
-    st = e == cudaSuccess ? ae_rt_synchronize(rc->ctx, nullptr) : CudaFail(rc->ctx, e, "self-test launch");
-    cudaFree(out);
-    if (st == AE_RT_TIMEOUT) {
-        *timed_out = 1;
-        return AE_RT_OK;
+    uint32_t gave_up = 0;
+    for (int train = 0; train < 2 && st == AE_RT_OK; train++) {
+        // (the training kernel gives up before it adds anything to the gradients)
+        if (train) rc_train_tc_kernel<<<1, RCTT_THREADS, RCTT_SMEM>>>(p);
+        else rc_infer_tc_kernel<RC_PREDICT><<<1, RCT_THREADS, RCT_SMEM>>>(p);
+        const cudaError_t e = cudaGetLastError();
+        st = e == cudaSuccess ? ae_rt_synchronize(rc->ctx, nullptr) : CudaFail(rc->ctx, e, "self-test launch");
+        if (st == AE_RT_TIMEOUT) {
+            gave_up++;
+            st = AE_RT_OK;
+        }
     }
+    cudaFree(out);
+    *timed_out = gave_up == 2 ? 1u : 0u;
     return st;
 }
 

@@ -572,7 +572,7 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
 #pragma unroll 1
             for (int l = 0; l <= RC_HIDDEN && ok; l++) {
                 const uint32_t nn = l < RC_HIDDEN ? uint32_t(RC_W) : uint32_t(RC_OUT);
-                if (row == 0) {
+                if (row == 0 && !p.skip_mma) {
                     const uint32_t idesc = rct_idesc(RC_TILE, nn);
 #pragma unroll
                     for (uint32_t s = 0; s < 4; s++)
@@ -712,7 +712,12 @@ static __global__ void __launch_bounds__(RCTT_THREADS, 1) rc_train_tc_kernel(RcM
             const uint32_t b = k & 1u;
             if (k >= 2) {
                 const uint32_t kk = k - 2;
-                if (!mbar_wait(grads_bar(b), (kk >> 1) & 1u)) { *fail = 1u; ok = false; break; }
+                // one decision per warp: the scatter's shuffles take all of its lanes
+                if (!__all_sync(0xffffffffu, mbar_wait(grads_bar(b), (kk >> 1) & 1u))) {
+                    *fail = 1u;
+                    ok = false;
+                    break;
+                }
                 const uint32_t gi = (blockIdx.x + kk * gridDim.x) * RC_TILE + row;
                 const bool valid = gi < count;
                 const float4 q0 = valid ? p.recs[size_t(first + gi) * 4] : make_float4(0, 0, 0, 0);
