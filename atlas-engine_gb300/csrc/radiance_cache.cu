@@ -3,6 +3,7 @@
 // paths, rendering with paths terminated into the cache.
 #include "atlas_rt.h"
 #include "context.cuh"
+#include "direct_output.h"
 #include "rc_kernels.cuh"
 #include "rc_tc_kernels.cuh"
 
@@ -576,12 +577,19 @@ ae_rt_status ae_rc_gradients(ae_rc* rc, const float* samples, uint32_t n, float*
     if (n == 0 || !DevPtr(samples)) return RcFail(rc, AE_RT_INVALID_ARG, "ae_rc_gradients takes device samples");
     RC_CUDA(rc, cudaSetDevice(rc->ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // into the caller's device buffers at once where their alignment lets the
-    // kernel add in 16 bytes (through the cache's own, 2 x 67 MB of copy at 2^19
-    // entries a level)
-    auto direct = [](float* g) { return g && DevPtr(g) && (reinterpret_cast<uintptr_t>(g) & 15u) == 0 ? g : nullptr; };
-    float* const mlp_out = direct(grad_mlp);
-    float* const grid_out = direct(grad_grid);
+    // into the caller's device buffers at once where the kernels may write them
+    // (through the cache's own, 2 x 67 MB of copy at 2^19 entries a level)
+    auto direct = [&](float* g, size_t params) -> float* {
+        cudaPointerAttributes a{};
+        if (!g) return nullptr;
+        if (cudaPointerGetAttributes(&a, g) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return DirectOutput(a, rc->ctx->device, g, params * sizeof(float), samples, size_t(n) * 64) ? g : nullptr;
+    };
+    float* const mlp_out = direct(grad_mlp, RC_NPARAM);
+    float* const grid_out = direct(grad_grid, rc->grid_params);
     ae_rt_status st = Backprop(rc, reinterpret_cast<const float4*>(samples), n, nullptr, 0, 0, s, mlp_out, grid_out);
     if (st != AE_RT_OK) return st;
     if (grad_mlp && !mlp_out)
