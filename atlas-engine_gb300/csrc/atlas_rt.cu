@@ -279,10 +279,10 @@ uint32_t atlas::rt::host::GridFor(const ae_rt_ctx* ctx, const void* fn, uint32_t
 }
 
 cudaError_t atlas::rt::host::NextWorkCounter(ae_rt_ctx* ctx, cudaStream_t s, uint32_t** counter) {
-    constexpr uint32_t kWorkSlots = 6;
+    // words 0 and 1 hold the error word; two words a slot behind them
     const uint32_t k = ctx->next_work_slot++ % kWorkSlots;
-    *counter = ctx->d_counter + (k == 0 ? 0u : k + 1u);      // word 1 is the error word
-    return cudaMemsetAsync(*counter, 0, sizeof(uint32_t), s);
+    *counter = ctx->d_counter + 2 + 2 * k;
+    return cudaMemsetAsync(*counter, 0, 2 * sizeof(uint32_t), s);
 }
 
 namespace {
@@ -527,8 +527,9 @@ ae_rt_status ae_rt_ctx_create(const ae_rt_config* cfg, ae_rt_ctx** out) {
     if (c.refill_below > 0 && c.refill_below <= 32) ctx->refill_steps = std::min(ctx->refill_steps, 8u);
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, 8 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, 8 * sizeof(uint32_t));
+    constexpr size_t counter_bytes = (2 + 2 * kWorkSlots) * sizeof(uint32_t);
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, counter_bytes);
+    if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, counter_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_fetch, 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_fetch, 0, 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_cast_counts, 4 * sizeof(uint32_t));
@@ -846,8 +847,8 @@ ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32
     return AE_RT_OK;
 }
 
-// The batched launch over a device copy of `t.desc`; counters: two words;
-// count: fetch totals.
+// The batched launch over a device copy of `t.desc`; counters: two zeroed
+// words; count: fetch totals.
 cudaError_t LaunchBatches(ae_rt_ctx* ctx, const BatchTable& t, const atlas::rt::dev::BatchDesc* d_desc,
                           uint32_t* counters, bool count, cudaStream_t s) {
     TraceParams p[2] = {};
@@ -862,8 +863,6 @@ cudaError_t LaunchBatches(ae_rt_ctx* ctx, const BatchTable& t, const atlas::rt::
         p[any].spread_warps = SpreadWarps(ctx);
         p[any].max_steps = 0xffffffffu;
     }
-    cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
     void* fn = PickBatch(ctx->shape, t.depth, count, ctx->near_ties);
     void* args[] = { &p[0], &p[1] };
     const size_t stacks = size_t(ctx->threads) * size_t(kShapes[ctx->shape].smem) * sizeof(int32_t);
@@ -882,14 +881,16 @@ ae_rt_status ae_rt_trace_batched(ae_rt_ctx* ctx, const ae_batch_desc* batches, u
     if (st != AE_RT_OK) return st;
     if (t.rays[0] + t.rays[1] == 0) return AE_RT_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // the table, then the two work counters
     const size_t bytes = t.desc.size() * sizeof(t.desc[0]);
-    AE_CUDA(ctx, ctx->batch_table.ensure(bytes + 2 * sizeof(uint32_t)));
+    AE_CUDA(ctx, ctx->batch_table.ensure(bytes));
     auto* d_desc = static_cast<atlas::rt::dev::BatchDesc*>(ctx->batch_table.ptr);
     AE_CUDA(ctx, cudaMemcpyAsync(d_desc, t.desc.data(), bytes, cudaMemcpyHostToDevice, s));
     if (ctx->count_fetches) AE_CUDA(ctx, cudaMemsetAsync(ctx->d_fetch, 0, 2 * sizeof(unsigned long long), s));
-    AE_CUDA(ctx, LaunchBatches(ctx, t, d_desc, reinterpret_cast<uint32_t*>(d_desc + t.desc.size()),
-                               ctx->count_fetches, s));
+    // counters of the launch's own: a launch of the same table on another
+    // stream may still be handing out its rays
+    uint32_t* counters = nullptr;
+    AE_CUDA(ctx, NextWorkCounter(ctx, s, &counters));
+    AE_CUDA(ctx, LaunchBatches(ctx, t, d_desc, counters, ctx->count_fetches, s));
     return AE_RT_OK;
 }
 
@@ -912,9 +913,9 @@ ae_rt_status ae_rt_batch_plan_create(ae_rt_ctx* ctx, const ae_batch_desc* batche
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const cudaError_t le = LaunchBatches(ctx, t, plan->d_batches,
-                                             reinterpret_cast<uint32_t*>(plan->d_batches + t.desc.size()), false,
-                                             cap);
+        auto* counters = reinterpret_cast<uint32_t*>(plan->d_batches + t.desc.size());
+        cudaError_t le = cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), cap);
+        if (le == cudaSuccess) le = LaunchBatches(ctx, t, plan->d_batches, counters, false, cap);
         e = cudaStreamEndCapture(cap, &plan->graph);
         if (le != cudaSuccess) e = le;
     }

@@ -113,7 +113,7 @@ struct ae_rt_ctx {
     atlas::rt::host::Scratch pass_rays, pass_key, pass_hits, pass_rad, pass_shadow, pass_shadow_pay, pass_vis,
         pass_counts;
     uint32_t* d_pt_counts = nullptr;    // radiance-cache render: [0], [1] ray queues, [2], [3] shadow queues
-    uint32_t* d_counter = nullptr;     // [1] error word; [0], [2..6] work counters (rotated per launch)
+    uint32_t* d_counter = nullptr;     // [1] error word; [2..] work counters, two a launch (kWorkSlots in rotation)
     uint32_t next_work_slot = 0;
     unsigned long long* d_fetch = nullptr;
     atlas::rt::host::Scratch rays_in, results_out, batch_table, retest_count;
@@ -162,8 +162,6 @@ inline bool IsDevicePointer(const void* p) {
 }
 
 
-// The work counter of the context's next persistent launch, zeroed on its
-// stream: six in rotation, so that launches on different streams can overlap.
 // Launches a kernel that begins with dev::wait_for_previous: it is set up while
 // the kernel before it on the stream drains, instead of after it has ended
 // (programmatic dependent launch).  The chains of short kernels gain most: a
@@ -194,6 +192,11 @@ cudaError_t LaunchNext(void (*kernel)(P...), uint32_t grid, uint32_t threads, cu
         },
         values);
 }
+
+// The work counters (two words; most launches use the first alone) of the
+// context's next persistent launch, zeroed on its stream: kWorkSlots in
+// rotation, so that launches on different streams can overlap.
+constexpr uint32_t kWorkSlots = 6;
 cudaError_t NextWorkCounter(ae_rt_ctx* ctx, cudaStream_t s, uint32_t** counter);
 
 // Persistent grid for kernel `fn`: SMs x resident CTAs (the configured count,
