@@ -722,9 +722,10 @@ static __device__ __noinline__ float texture_opacity(const float* materials, uin
 // below 1e-6 become 0, and the traversal ends at 0.
 //
 // FEW: the launch's warps hold all of its rays at once (the host has checked
-// the count), each warp its own range, so there is no work counter and no
-// memset before the launch (1,000 closest hits 39 -> 36 us; a test for it at
-// run time cost the large launches up to 3 %).
+// the count; the transparency queries launch as many blocks as that takes),
+// each warp its own range, so there is no work counter and no memset before
+// the launch (1,000 closest hits 39 -> 36 us; a test for it at run time cost
+// the large launches up to 3 %).
 //
 // CAMERA: ray i is the camera ray of queue slot i (camera_ray), made by the
 // lane that takes it, instead of a load from a ray buffer written by a
@@ -794,7 +795,7 @@ __device__ __forceinline__ void trace_rays(const TraceParams& p) {
     const uint32_t burst = p.refill_steps;
     // rays a warp holds at a time: all lanes, or its share of a small launch
     const uint32_t share = min(p.spread_warps, gridDim.x * uint32_t(WARPS));
-    const bool mayHold = lane < (nRays + share - 1) / share;
+    const bool mayHold = lane < (FEW ? (nRays - 1) / share + 1 : (nRays + share - 1) / share);
 
     // a ray's traversal state from its origin and direction (tmax already set)
     auto beginRay = [&](const float4& o4, const float4& d4, uint32_t nodesHere) {

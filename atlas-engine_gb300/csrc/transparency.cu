@@ -4,12 +4,14 @@
 //                           (+ CheckLeafClosestTransparency :106-138)
 //   HitAnyTransparency      data/shader/raytracer/bvh.hsh:443-524
 //                           (+ CheckLeafTransparency :140-170)
-// over the context's two-level scene: the OPACITY instances of the persistent
-// traversal kernel (trace_kernels.cuh).
+// over the context's two-level scene: the OPACITY instances of the traversal
+// kernel (trace_kernels.cuh).
 #include "atlas_rt.h"
 #include "context.cuh"
 #include "trace_kernels.cuh"
 #include "texture.cuh"
+
+#include <algorithm>
 
 using namespace atlas::rt::host;
 using namespace atlas::rt::dev;
@@ -22,10 +24,16 @@ namespace {
 // instead of 344 us).  The same frame took 393 us with one thread per ray and
 // a local-memory stack: a warp then kept its 32 rays to the end, and the
 // launch waited, 12 warps an SM and half of the SMs done, for the longest.
-template <bool ANY, int SPILL>
+template <bool ANY, int SPILL, bool FEW>
 void* KernelFor() {
     return reinterpret_cast<void*>(
-        &trace_kernel<ANY, false, MODE_SCENE, 4, 32, SPILL, 7, false, false, 0, false, false, true>);
+        &trace_kernel<ANY, false, MODE_SCENE, 4, 32, SPILL, 7, false, false, 0, false, false, true, FEW>);
+}
+
+template <bool FEW>
+void* Pick(bool any, bool shallow) {
+    return any ? (shallow ? KernelFor<true, 0, FEW>() : KernelFor<true, 96, FEW>())
+               : (shallow ? KernelFor<false, 0, FEW>() : KernelFor<false, 96, FEW>());
 }
 
 }  // namespace
@@ -82,14 +90,24 @@ ae_rt_status atlas::rt::host::TraceTransparency(ae_rt_ctx* ctx, bool any, const 
     p.transparency = any ? static_cast<float*>(d_out) : nullptr;
     p.error_word = ctx->d_counter + 1;
     p.work_counter = counter;
-    if (!counter) AE_CUDA(ctx, NextWorkCounter(ctx, s, &p.work_counter));
     p.refill_steps = ctx->refill_steps;
     p.spread_warps = SpreadWarps(ctx);
     const bool shallow = ctx->scene_depth < 32u;
-    void* fn = any ? (shallow ? KernelFor<true, 0>() : KernelFor<true, 96>())
-                   : (shallow ? KernelFor<false, 0>() : KernelFor<false, 96>());
+    // A caller's own queries take no work counter, of which a context has only
+    // a few in rotation: any number of them may be in flight, on as many
+    // streams, and captured ones beside their replays.  Each warp holds its rays
+    // once, in as many blocks as that takes.  (With a counter of the rotation,
+    // which the seventh launch in flight cleared under the first, and its memset:
+    // a ray that misses everything 7 us against 5, 58,000 random rays 58 / 55
+    // against 55 / 52, two million camera rays 297 / 269 against 291 / 282, two
+    // million random ones 420 / 404 against 548 / 551, closest / any.  Ranges of
+    // 2 to 16 rays a lane win back a part of the last and lose up to twice the
+    // time on the camera's.)
+    void* fn = counter ? Pick<false>(any, shallow) : Pick<true>(any, shallow);
+    uint32_t grid = GridFor(ctx, fn, n, 128);
+    if (!counter) grid = std::max(grid, n / 128 + (n % 128 ? 1u : 0u));
     void* args[] = { &p };
-    AE_CUDA(ctx, LaunchNext(static_cast<const void*>(fn), GridFor(ctx, fn, n, 128), 128, s, args));
+    AE_CUDA(ctx, LaunchNext(static_cast<const void*>(fn), grid, 128, s, args));
     if (!out_dev) AE_CUDA(ctx, cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, s));
     if (!out_dev || !rays_dev) return ae_rt_synchronize(ctx, stream);
     return AE_RT_OK;
