@@ -26,7 +26,8 @@ struct DeviceMesh {
 };
 
 // A node in the library's device order (load_node in trace_kernels.cuh) from
-// the engine's layout, and back.  padding0 is the node's `slow` word.
+// the engine's layout (ae_rt_mesh_get_bvh: back).  padding0 is the node's
+// `slow` word.
 struct PairedNode {
     uint32_t w[16];
 };
@@ -37,13 +38,6 @@ __host__ __device__ inline PairedNode PairNode(const ae_bvh_node& e) {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&e);
     for (int k = 0; k < 16; k++) p.w[k] = src[dev::engine_node_word(k)];
     return p;
-}
-
-__host__ __device__ inline ae_bvh_node UnpairNode(const PairedNode& p) {
-    ae_bvh_node e;
-    uint32_t* dst = reinterpret_cast<uint32_t*>(&e);
-    for (int k = 0; k < 16; k++) dst[dev::engine_node_word(k)] = p.w[k];
-    return e;
 }
 
 // Grow-only device scratch buffer.

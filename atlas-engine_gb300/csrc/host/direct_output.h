@@ -8,8 +8,8 @@
 
 namespace atlas::rt::host {
 
-// True when kernels on `device` may clear `out` and add to it 16 bytes at a
-// time: 16-byte aligned memory of that very device (another GPU's may not be
+// True when kernels on `device` may write `out`, 16 bytes and atomically too:
+// 16-byte aligned memory of that very device (another GPU's may not be
 // mapped, and managed pages may lie in host memory), apart from the input
 // that is read meanwhile.  a: the attributes of `out`.
 inline bool DirectOutput(const cudaPointerAttributes& a, int device, const void* out, size_t bytes, const void* in,
