@@ -795,7 +795,9 @@ __device__ __forceinline__ void trace_rays(const TraceParams& p) {
     const uint32_t burst = p.refill_steps;
     // rays a warp holds at a time: all lanes, or its share of a small launch
     const uint32_t share = min(p.spread_warps, gridDim.x * uint32_t(WARPS));
-    const bool mayHold = lane < (FEW ? (nRays - 1) / share + 1 : (nRays + share - 1) / share);
+    // (staged warps claim whole tiles, which a few lanes would work off one after
+    // the other: 1,000 closest hits on 65,536 triangles 740 instead of 142 us)
+    const bool mayHold = STAGE > 0 || lane < (FEW ? (nRays - 1) / share + 1 : (nRays + share - 1) / share);
 
     // a ray's traversal state from its origin and direction (tmax already set)
     auto beginRay = [&](const float4& o4, const float4& d4, uint32_t nodesHere) {
