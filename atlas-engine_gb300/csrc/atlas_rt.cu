@@ -834,7 +834,6 @@ ae_rt_status MakeBatchTable(ae_rt_ctx* ctx, const ae_batch_desc* batches, uint32
             d.n_nodes = m.n_nodes;
             d.n_tris = m.n_tris;
             d.n_rays = b.n_rays;
-            d.any = uint32_t(any);
             d.tmin = b.tmin;
             d.tmax = b.tmax;
             d.first = t.rays[any];

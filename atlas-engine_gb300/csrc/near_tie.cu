@@ -34,7 +34,9 @@ constexpr uint32_t kRetestStack = 128;
 constexpr int kRetestSmem = 32;            // of them in shared memory
 constexpr int kRetestThreads = 128;
 constexpr int kRetestBlocks = 4;           // CTAs an SM
-constexpr int kRetestBatch = 4;            // lanes that test their triangles together
+// Lanes that test their triangles together: with 1, 2, 4, 8 and 16 of them a
+// 961 x 541 camera trace and its re-test take 547, 500, 482, 479 and 480 us.
+constexpr int kRetestBatch = 4;
 constexpr double kSecondWindow = 1e-5;     // ten times the 1e-6 of a near tie
 
 // The farthest distance that can still matter: best + |best| kSecondWindow

@@ -89,8 +89,8 @@ struct TraceParams {
     CameraParams cam;            // the camera variant: ray i is camera_ray(cam, i), `rays` unused
 };
 
-// One ray batch of a batched launch: its mesh, its rays and results, its
-// query kind, and its first index in the launch's global ray numbering.
+// One ray batch of a batched launch: its mesh, its rays and results, and its
+// first index in the global ray numbering of its query kind.
 struct BatchDesc {
     const float4* nodes;
     const float4* tris;
@@ -99,7 +99,7 @@ struct BatchDesc {
     uint32_t n_nodes;
     uint32_t n_tris;
     uint32_t n_rays;
-    uint32_t any;
+    uint32_t reserved;
     float tmin;
     float tmax;
     uint32_t first;              // global index of the batch's first ray
