@@ -48,8 +48,8 @@ sys.path.insert(0, str(REPO / "atlas-engine_gb300"))
 
 W, H = 1920, 1080
 # DRAM bytes (read + write) of the primary closest-hit launch of this workload
-# (camera rays made in the kernel), from ncu (31,899,392 + 18,045,952)
-TRAFFIC_PRIMARY_BYTES = 49_945_344
+# (camera rays made in the kernel), from ncu (31,911,424 + 17,654,528)
+TRAFFIC_PRIMARY_BYTES = 49_565_952
 TMIN, TINF = 0.0, 1e12
 EPSILON = 0.1
 LIGHT = (0.4, 1.0, 0.3)
@@ -357,11 +357,11 @@ def timed_steps(torch, dev, stream, step, steps, flush):
 # DRAM bytes (read + write) per launch from one ncu capture per ray class
 # (bench.py --profile cast / random65536 / batched64; profiles/trace_kernel_ray_classes.md)
 TRAFFIC_BYTES = {"primary": TRAFFIC_PRIMARY_BYTES,
-                 "bounce": 92_501_248 + 11_122_176,
-                 "shadow": 53_865_216 + 85_760,
-                 "random65536_closest": 57_699_072 + 4_891_392,
-                 "random65536_any": 57_689_088 + 346_624,
-                 "batched64": 1_200_891_136 + 263_677_952}
+                 "bounce": 92_505_600 + 10_715_648,
+                 "shadow": 53_864_960 + 73_728,
+                 "random65536_closest": 57_692_160 + 3_951_360,
+                 "random65536_any": 57_689_088 + 96_512,
+                 "batched64": 1_202_822_912 + 285_040_896}
 
 
 def class_roofline(alg_bytes, ms, hbm_peak, l2_gbs, traffic=None):
@@ -1366,9 +1366,9 @@ def main():
                      "traffic": tr["traffic"],
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of this launch, one ncu "
                                        "capture (profiles/)",
-                     "limiter": "instruction issue: ncu shows 72-80 % issue-active with not_selected the top "
-                                "stall, L2 throughput ~5 %, DRAM traffic a few % of the algorithmic bytes "
-                                "(the 59 MB BVH stays in the 129 MB L2)",
+                     "limiter": "instruction issue and load latency: ncu shows 63-66 % issue-active with "
+                                "long_scoreboard the top stall and not_selected next, L2 throughput 5-7 %, DRAM "
+                                "traffic a few % of the algorithmic bytes (the 59 MB BVH stays in the 129 MB L2)",
                      "note": "frac is against the measured HBM copy peak, as the contract asks; the node and "
                              "triangle bytes come from L2, so l2_frac (against an L2-resident copy measured in "
                              "the same run) is the meaningful bytes fraction",
